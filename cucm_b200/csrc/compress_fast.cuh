@@ -84,7 +84,7 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
   L.off_fr = take((size_t)2 * U * kOrders);                // frozen state
   L.off_yw = take(sizeof(uint32_t) * 4 * (U / 32));        // bits, by unit mod 4
   L.off_c1 = take((size_t)4 * (U / 8));                    // previous byte per byte, by unit mod 4
-  L.off_prm = take(sizeof(uint16_t) * 2 * U);              // coder input, by unit parity
+  L.off_prm = take(sizeof(uint2) * 2 * U);                 // coder input, by unit parity
   L.off_win = take((size_t)kWinBytes);
   L.off_stage = take((size_t)L.stage);
   L.total = o;
@@ -105,7 +105,7 @@ struct FastSmem {
   uint8_t *fr;       // [2][U][8]
   uint32_t *yw;      // [4][U/32]
   uint8_t *c1;       // [4][U/8]
-  uint16_t *prm;     // [2][U]
+  uint2 *prm;        // [2][U]
   uint8_t *win;      // [kWinBytes]
   uint8_t *stage;
 };
@@ -125,7 +125,7 @@ __device__ inline FastSmem carve_fast(uint8_t *b, const FastLayout &L) {
   s.fr = b + L.off_fr;
   s.yw = reinterpret_cast<uint32_t *>(b + L.off_yw);
   s.c1 = b + L.off_c1;
-  s.prm = reinterpret_cast<uint16_t *>(b + L.off_prm);
+  s.prm = reinterpret_cast<uint2 *>(b + L.off_prm);
   s.win = b + L.off_win;
   s.stage = b + L.off_stage;
   return s;
@@ -454,8 +454,8 @@ __device__ __forceinline__ void front_mix(const FastSmem &s, const FastLayout &L
   const int U = L.U;
   const uint32_t *yw = s.yw + (v & 3) * (U / 32);
   const uint8_t *c1 = s.c1 + (v & 3) * (U / 8);
-  uint16_t *prm = s.prm + (v & 1) * U;
-  const uint16_t *prm_old = s.prm + ((v + 1) & 1) * U;
+  uint2 *prm = s.prm + (v & 1) * U;
+  const uint2 *prm_old = s.prm + ((v + 1) & 1) * U;
   int cxs[2] = {0, 0}, errs[2] = {0, 0};
   bool has[2] = {false, false};
   CUCM_UNROLL
@@ -469,7 +469,7 @@ __device__ __forceinline__ void front_mix(const FastSmem &s, const FastLayout &L
         const int cx = olen + (c1[j >> 3] >> 5) * 10;
         const int pr = mix_pr(s.w, cx, smps[h], s.tab);
         const int y = (yw[j >> 5] >> (j & 31)) & 1;
-        prm[j] = (uint16_t)((pr << 1) | y);
+        prm[j] = coder_entry((uint32_t)((pr << 1) | y));
         cxs[h] = cx;
         errs[h] = ((y << 12) - pr) * 7;
         has[h] = true;
@@ -556,7 +556,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
     s.rec[i] = (uint64_t)v | ((uint64_t)s.tab->dt[c] << 32) | ((uint64_t)s.tab->dt[c < 1023u ? c + 1 : 1023u] << 48);
   }
   for (int i = tid; i < kMixCtx * kOrders; i += blockDim.x) s.w[i] = init->w[i];
-  for (int i = tid; i < 2 * U; i += blockDim.x) s.prm[i] = 0;  // cucm_compress_v2.cu:1039-1040
+  for (int i = tid; i < 2 * U; i += blockDim.x) s.prm[i] = coder_entry(0);  // cucm_compress_v2.cu:1039-1040
   for (int i = tid; i < 2 * kOrders * L.NSLOT; i += blockDim.x) s.hk[i] = 0;
 
   Coder c{0u, 0xffffffffu, 0, 0};
@@ -622,7 +622,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
   }
 
   if (warp == kWCoder) {
-    const uint16_t *last = s.prm + ((nU - 1) & 1) * U;
+    const uint2 *last = s.prm + ((nU - 1) & 1) * U;
     const uint64_t coded = (uint64_t)nU * U;
     const uint64_t left = total_bits > coded ? total_bits - coded : 0;
     if (tails && left >= kTailOffloadBits) {
@@ -636,7 +636,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
       if (lane == 0) k = atomicAdd(tail_count, 1u);
       k = __shfl_sync(0xffffffffu, k, 0);
       TailTask &T = tails[k];
-      for (int j = lane; j < U; j += 32) T.prm[j] = last[j];
+      for (int j = lane; j < U; j += 32) T.prm[j] = (uint16_t)coder_entry_u16(last[j]);
       if (lane == 0) {
         T.out = t.out;
         T.cap = t.out_cap;
@@ -731,44 +731,42 @@ __global__ void __launch_bounds__(kFastThreads, 2)
 
 // The tail pass: one thread per handed-over chunk codes its stale tail (the
 // unit buffer again and again up to the chunk end), writes the bytes, the
-// flush byte (cucm_compress_v2.cu:902) and the payload length.  Same coder
-// step as coder_step; the buffer is read through the read-only cache, four
-// entries per load.
-__global__ void __launch_bounds__(128) compress_tail_kernel(const TailTask *tails, const uint32_t *count,
-                                                            uint32_t *status) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= *count) return;
+// flush byte (cucm_compress_v2.cu:902) and the payload length.  `lanes`
+// chunks share a warp, each with its unit buffer in a row of shared memory
+// (rows 16 bytes apart in the banks).
+// One 20 KB buffer at 1 MiB chunks (8.2 million stale bits): 424 -> 260 ms
+// against a test after every bit.
+inline size_t tail_smem_bytes(int unit, int lanes) {
+  return (size_t)lanes * ((size_t)(unit + 2) * sizeof(uint2) + kLaneRing + 4);
+}
+
+__global__ void __launch_bounds__(32) compress_tail_kernel(const TailTask *tails, const uint32_t *count,
+                                                           uint32_t *status, int unit, int lanes) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int lane = threadIdx.x;
+  const uint32_t i = blockIdx.x * (uint32_t)lanes + lane;
+  if (lane >= lanes || i >= *count) return;
   const TailTask &T = tails[i];
+  uint2 *ent = reinterpret_cast<uint2 *>(smem_raw) + (unit + 2) * lane;
+  uint8_t *ring = lane_ring(smem_raw + (size_t)(unit + 2) * lanes * sizeof(uint2), lane);
+  for (int j = 0; j < unit; j++) ent[j] = coder_entry(T.prm[j]);
   uint32_t x1 = T.x1, x2 = T.x2;
-  uint64_t head = T.head;
   const uint64_t cap = T.cap;
+  uint64_t base = T.head;  // payload offset of ring position 0
   uint8_t *out = T.out;
-  const uint32_t U = T.unit;
-  const uint64_t *prm4 = reinterpret_cast<const uint64_t *>(T.prm);
+  uint32_t head = 0, from = 0;  // bytes since base: produced, written
   uint64_t left = T.bits;
-  uint32_t j4 = 0;  // next group of four entries
-  while (left) {
-    const uint64_t e4 = __ldg(prm4 + j4);
-    j4 = (4 * (j4 + 1) == U) ? 0u : j4 + 1;
-    const int n = left < 4 ? (int)left : 4;
-    left -= (uint64_t)n;
-CUCM_UNROLL
-    for (int q = 0; q < 4; q++) {
-      if (q < n) {
-        const uint32_t e = (uint32_t)(e4 >> (16 * q)) & 0xffffu;
-        const uint32_t xm = x1 + __umulhi(x2 - x1, (e >> 1) << 20);
-        if (e & 1) x2 = xm; else x1 = xm + 1;
-        while ((x1 ^ x2) < 0x1000000u) {
-          if (head < cap) out[head] = (uint8_t)(x2 >> 24);
-          head++;
-          x1 <<= 8;
-          x2 = (x2 << 8) | 255u;
-        }
-      }
-    }
+  int j = 0;
+  for (; left >= kCoderGroup; left -= kCoderGroup) {
+    coder_group_at(ent + j, x1, x2, head, ring, kLaneRing - 1);
+    j = j + kCoderGroup == unit ? 0 : j + kCoderGroup;
+    if (lane_flush_due(from, head)) lane_flush(ring, base, from, head, out, cap);
   }
-  if (head < cap) out[head] = (uint8_t)(x1 >> 24);
+  for (int k = 0; k < (int)left; k++) coder_step(ent[j + k], x1, x2, head, ring, kLaneRing - 1);
+  ring[head & (kLaneRing - 1)] = (uint8_t)(x1 >> 24);
   head++;
-  *T.result = head;
-  if (head > cap) atomicOr(status, (uint32_t)kDevOverflow);
+  lane_flush(ring, base, from, head, out, cap);
+  base += head;  // (what is left of the last ring)
+  *T.result = base;
+  if (base > cap) atomicOr(status, (uint32_t)kDevOverflow);
 }

@@ -178,7 +178,14 @@ __device__ inline void write_back(const Smem &s, const Layout &L, uint8_t *slot)
 }
 
 __device__ inline void coder_run(Coder &c, const Smem &s, const Layout &L, int n) {
-  coder_run_p(c, s.prm, s.stage, L.stage, n);
+  auto entry = [&](int j) { return coder_entry(s.prm[j]); };
+  coder_run(
+      c, s.stage, L.stage, n,
+      [&](int j, uint32_t &x1, uint32_t &x2, uint32_t &head, uint32_t mask) {
+        auto at = [&](int k) { return entry(j + k); };
+        coder_group(at, at, x1, x2, head, s.stage, mask);
+      },
+      entry);
 }
 __device__ inline void coder_flush_blocks(Coder &c, const Smem &s, const Layout &L, uint8_t *out, uint64_t cap) {
   coder_flush_p(c, s.stage, L.stage, out, cap);
@@ -552,6 +559,16 @@ size_t decompress_smem_bytes(int unit, int spec_bits) {
   return make_layout(unit, 0).total + kNodeBytes;
 }
 
+// Chunks that share a warp of a one-thread-per-chunk coder kernel: one while
+// every chunk can have a warp scheduler of its own (a group that is done again
+// for one lane holds up the warp's others), else just enough.
+static int coder_lanes(uint32_t ntasks, int sm_count) {
+  const uint32_t warps = 4u * (uint32_t)(sm_count > 0 ? sm_count : 148);
+  int lanes = 1;
+  while (lanes < 32 && (ntasks + lanes - 1) / lanes > warps) lanes *= 2;
+  return lanes;
+}
+
 cudaError_t launch_fixed_encode(const FixedTask *d_tasks, const uint64_t *d_first, uint32_t ntasks, uint64_t total,
                                 const uint8_t *image, const ModelInit *d_init, uint32_t *d_status, int sm_count,
                                 cudaStream_t stream) {
@@ -564,8 +581,8 @@ cudaError_t launch_fixed_encode(const FixedTask *d_tasks, const uint64_t *d_firs
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  // one warp of coders per CTA: the warps land on different SMs
-  fixed_coder_kernel<<<(ntasks + 31) / 32, 32, 0, stream>>>(d_tasks, ntasks, d_status);
+  const int lanes = coder_lanes(ntasks, sm_count);
+  fixed_coder_kernel<<<(ntasks + lanes - 1) / lanes, 32, 0, stream>>>(d_tasks, ntasks, d_status, lanes);
   return cudaGetLastError();
 }
 
@@ -620,7 +637,11 @@ cudaError_t launch_compress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t *
                                                                          d_queue, d_status, unit, tails, tail_count);
     e = cudaGetLastError();
     if (e != cudaSuccess || !tails) return e;
-    compress_tail_kernel<<<(ntasks + 127) / 128, 128, 0, stream>>>(tails, tail_count, d_status);
+    const int lanes = coder_lanes(ntasks, cfg.sm_count);
+    const size_t tsmem = tail_smem_bytes(unit, lanes);
+    e = set_smem((const void *)compress_tail_kernel, tsmem);
+    if (e != cudaSuccess) return e;
+    compress_tail_kernel<<<(ntasks + lanes - 1) / lanes, 32, tsmem, stream>>>(tails, tail_count, d_status, unit, lanes);
     return cudaGetLastError();
   }
   const size_t smem = make_layout(unit, 0).total;
