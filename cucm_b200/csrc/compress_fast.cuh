@@ -10,13 +10,12 @@
 // itself:
 //
 //   front warps (3..6, 128 threads)
-//     * keys of unit t+2 for all 8 orders (one FNV pass per bit,
+//     * keys of unit t+1 for all 8 orders (one FNV pass per bit,
 //       cucm_compress_v2.cu:723-747), the unit's bits and previous bytes;
-//     * slot links of unit t+1: per order, the unit's keys sorted across a
-//       warp give every distinct slot of the unit one place (its first
-//       position), so every later touch knows it must read the state its
-//       predecessor left; a binary search of the previous unit's sorted keys
-//       tells whether the slot was touched one unit earlier;
+//     * slot links of unit t+1: per order, bits that touch the same slot share
+//       one number, so every later touch knows it must read the state its
+//       predecessor left, and know whether the slot was touched one unit
+//       earlier;
 //     * gathers of unit t+1's slot states from the tables in HBM;
 //     * stretch, mixer context, mixer output and training of unit t-1
 //       (cudamixUnit / cudaupdateMixer, cucm_compress_v2.cu:755-819) against
@@ -52,16 +51,22 @@ constexpr int kFastStageMin = 2048;
 // slower: the lookups are on the front warps' critical path).
 typedef Tables FastTables;
 
+constexpr uint32_t kUntouched = 0xffu;  // no state: the largest is 252
+constexpr int kClaimLog = 9, kClaim = 1 << kClaimLog;  // places of a claim table
+
 struct FastLayout {
   int U, NSLOT, stage;
-  size_t off_tab, off_rec, off_w, off_hk, off_ns, off_key, off_lnk, off_bkt, off_fsw, off_st, off_fr,
+  int ks, ls;   // row lengths of key and of lnk / bkt
+  size_t off_tab, off_rec, off_w, off_claim, off_late, off_ns, off_key, off_lnk, off_bkt, off_fsw, off_st, off_fr,
       off_yw, off_c1, off_prm, off_win, off_stage, total;
 };
 
 __host__ __device__ inline FastLayout make_fast_layout(int U) {
   FastLayout L;
   L.U = U;
-  L.NSLOT = U <= 128 ? 128 : 256;  // slots per order and unit: the keys sorted in 4 or 8 per lane
+  L.NSLOT = U <= 128 ? 128 : 256;  // slots per order and unit
+  L.ks = U + 4;  // rows of 8 orders that start in different banks
+  L.ls = U + 8;
   L.stage = next_pow2(4 * U + 1024);  // a unit codes at most 4U bytes; flushes go out in 512-byte blocks
   if (L.stage < kFastStageMin) L.stage = kFastStageMin;
   const size_t NS = (size_t)L.NSLOT;
@@ -74,11 +79,12 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
   L.off_tab = take(sizeof(FastTables));
   L.off_rec = take(sizeof(uint64_t) * kOrders * 256);
   L.off_w = take(sizeof(int32_t) * kMixCtx * kOrders);
-  L.off_hk = take(sizeof(uint32_t) * 2 * kOrders * NS);    // keys + 1 by slot, ascending [unit parity][order][slot]
-  L.off_ns = take(sizeof(uint16_t) * 2 * kOrders * NS);    // 0x100 | state once written in the unit
-  L.off_key = take(sizeof(uint32_t) * 2 * kOrders * U);    // [unit parity][bit][order]
-  L.off_lnk = take(sizeof(uint16_t) * 2 * kOrders * U);    // slot + 1 in the previous unit's table, or 0
-  L.off_bkt = take(sizeof(uint16_t) * 2 * kOrders * U);    // slot in this unit's table
+  L.off_claim = take((size_t)2 * kOrders * 2 * kClaim);   // claim tables [unit parity][order][round]
+  L.off_late = take((size_t)2 * kOrders * (NS + 4));       // slots claimed after the rounds [unit parity][order]
+  L.off_ns = take((size_t)2 * kOrders * NS);               // state written in the unit, or kUntouched
+  L.off_key = take(sizeof(uint32_t) * 2 * kOrders * L.ks); // [unit parity][order][bit]
+  L.off_lnk = take(sizeof(uint16_t) * 2 * kOrders * L.ls); // slot + 1 in the previous unit, or 0 [unit parity][order][bit]
+  L.off_bkt = take((size_t)2 * kOrders * L.ls);            // slot in this unit
   L.off_fsw = take((size_t)2 * kOrders * U);               // gathered slot states
   L.off_st = take((size_t)2 * kOrders * U + 4 * kOrders);  // live state (+ the chain's read-ahead)
   L.off_fr = take((size_t)2 * U * kOrders);                // frozen state
@@ -95,11 +101,12 @@ struct FastSmem {
   FastTables *tab;
   uint64_t *rec;     // [256][8]  statep | dt[count] << 32 | dt[count + 1] << 48
   int32_t *w;        // [80*8]
-  uint32_t *hk;      // [2][8][NSLOT]
-  uint16_t *ns;      // [2][8][NSLOT]
-  uint32_t *key;     // [2][U][8]
-  uint16_t *lnk;     // [2][U][8]
-  uint16_t *bkt;     // [2][U][8]
+  uint8_t *claim;    // [2][8][2][kClaim]
+  uint8_t *late;     // [2][8][NSLOT + 4]: count, slots
+  uint8_t *ns;       // [2][8][NSLOT]
+  uint32_t *key;     // [2][8][ks]
+  uint16_t *lnk;     // [2][8][ls]
+  uint8_t *bkt;      // [2][8][ls]
   uint8_t *fsw;      // [2][U][8]
   uint8_t *st;       // [2][U][8]
   uint8_t *fr;       // [2][U][8]
@@ -115,11 +122,12 @@ __device__ inline FastSmem carve_fast(uint8_t *b, const FastLayout &L) {
   s.tab = reinterpret_cast<FastTables *>(b + L.off_tab);
   s.rec = reinterpret_cast<uint64_t *>(b + L.off_rec);
   s.w = reinterpret_cast<int32_t *>(b + L.off_w);
-  s.hk = reinterpret_cast<uint32_t *>(b + L.off_hk);
-  s.ns = reinterpret_cast<uint16_t *>(b + L.off_ns);
+  s.claim = b + L.off_claim;
+  s.late = b + L.off_late;
+  s.ns = b + L.off_ns;
   s.key = reinterpret_cast<uint32_t *>(b + L.off_key);
   s.lnk = reinterpret_cast<uint16_t *>(b + L.off_lnk);
-  s.bkt = reinterpret_cast<uint16_t *>(b + L.off_bkt);
+  s.bkt = b + L.off_bkt;
   s.fsw = b + L.off_fsw;
   s.st = b + L.off_st;
   s.fr = b + L.off_fr;
@@ -154,7 +162,7 @@ __device__ __forceinline__ uint32_t window_load(const uint8_t *in, uint64_t len,
 // Front: keys, bits and previous bytes of unit v from the staged window.
 __device__ __forceinline__ void front_keys(const FastSmem &s, const FastLayout &L, int t, int v, int nvalid) {
   const int U = L.U;
-  uint32_t *key = s.key + (v & 1) * kOrders * U;
+  uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
   uint32_t *yw = s.yw + (v & 3) * (U / 32);
   uint8_t *c1 = s.c1 + (v & 3) * (U / 8);
   for (int j0 = 0; j0 < U; j0 += kFrontThreads) {
@@ -175,9 +183,8 @@ __device__ __forceinline__ void front_keys(const FastSmem &s, const FastLayout &
         acc = (acc ^ (uint32_t)s.win[q + 7 - o]) * kFnvPrime;
         k8[o] = acc & (kSlots - 1);
       }
-      uint4 *dst = reinterpret_cast<uint4 *>(key + j * kOrders);
-      dst[0] = make_uint4(k8[0], k8[1], k8[2], k8[3]);
-      dst[1] = make_uint4(k8[4], k8[5], k8[6], k8[7]);
+      CUCM_UNROLL
+      for (int o = 0; o < kOrders; o++) key[o * L.ks + j] = k8[o];
       y = (cur >> (7 - r)) & 1u;
       if (r == 0) c1[q] = (uint8_t)p1;
     }
@@ -187,106 +194,145 @@ __device__ __forceinline__ void front_keys(const FastSmem &s, const FastLayout &
   }
 }
 
-// Slot tables: per order and unit, the unit's keys (key + 1) in ascending
-// order, padded with kNoKey; a key's slot is the position of its first
-// occurrence.  Sorting the unit's keys once replaces a hash table built step
-// by step (a claim loop with a shared-memory round trip and a warp barrier
-// per two bytes); keeping the repeats in the row (slots with gaps) saves the
-// compaction.
-constexpr uint32_t kNoKey = 0xffffffffu;
-
-// Ascending bitonic sort of 32 * E values, value p = lane * E + i in a[i]
-// of lane `lane`: distances below E are compare-swaps within a lane, the
-// others exchange with lane ^ (distance / E) by shuffle.
-template <int E>
-__device__ __forceinline__ void warp_sort(uint32_t (&a)[E], int lane) {
-  constexpr int N = 32 * E;
-  CUCM_UNROLL
-  for (int k = 2; k <= N; k <<= 1) {
-    CUCM_UNROLL
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j >= E) {
-        const int lm = j / E;
-        const bool lower = (lane & lm) == 0;
-        CUCM_UNROLL
-        for (int i = 0; i < E; i++) {
-          const uint32_t o = __shfl_xor_sync(0xffffffffu, a[i], lm);
-          const bool up = ((lane * E + i) & k) == 0;
-          a[i] = (up == lower) ? min(a[i], o) : max(a[i], o);
-        }
-      } else {
-        CUCM_UNROLL
-        for (int i = 0; i < E; i++) {
-          if ((i & j) == 0) {
-            const bool up = ((lane * E + i) & k) == 0;
-            const uint32_t x = a[i], y = a[i | j];
-            a[i] = up ? min(x, y) : max(x, y);
-            a[i | j] = up ? max(x, y) : min(x, y);
-          }
-        }
-      }
-    }
-  }
-}
-
-// First position of kp in an ascending row of P (a power of two) entries,
-// if it is there: the returned position holds kp exactly when it is present.
-template <int P>
-__device__ __forceinline__ int row_find(const uint32_t *row, uint32_t kp) {
-  int lo = 0;
-  CUCM_UNROLL
-  for (int step = P >> 1; step > 0; step >>= 1) lo += row[lo + step - 1] < kp ? step : 0;
-  return lo;
-}
-
-// Front: slots of unit v in its own table, and in the previous unit's.
+// Slots of a unit: per order, bits that touch the same table slot share one
+// number, the position of one of them, and a bit whose slot the previous unit
+// touched too knows that unit's number for it.
+//
+// Every bit writes its position to a small claim table at a hash of its key;
+// whoever's position is there afterwards is the slot's number for all bits
+// with that key (they all hash to the same place), and bits that find another
+// key's claim go on to a second table.  Nothing is cleared: a place is only
+// read by bits that have just written it, and the previous unit's tables only
+// lead to a position whose key is compared.  With 4 places per bit (units of
+// 128 bits), 12 % of the keys need the second table and one in ~600 neither
+// claim: those are numbered one after the other and listed.  The two orders' ~12 shared-memory steps take
+// 3,250 cycles a unit of 128 bits for a CTA alone; sorting each order's keys
+// across the warp and searching the rows took 8,100 of the front warps'
+// 12,000.
+//
 // Front warp w owns orders 2w and 2w + 1, so no other warp writes their
-// rows.  Per order: the unit's keys (bit j = lane + 32 i) are sorted across
-// the warp and written in order, then every bit finds its key's first
-// position in this unit's row (bkt) and in the previous unit's (lnk =
-// position + 1, or 0 when the key was not touched there).  E keys per
-// lane: 32 * E >= U, and NSLOT = 32 * E.
+// tables.  E bits per lane: 32 * E >= U.
+__device__ __forceinline__ uint32_t claim_at(uint32_t key, int round, int logn) {
+  return (key * (round ? 0x85EBCA6Bu : 0x9E3779B1u)) >> (32 - logn);
+}
+
 template <int E>
 __device__ __forceinline__ void front_links(const FastSmem &s, const FastLayout &L, int t, int v, int nvalid) {
-  constexpr int P = 32 * E;
-  const int U = L.U;
-  const uint32_t *key = s.key + (v & 1) * kOrders * U;
-  uint16_t *lnk = s.lnk + (v & 1) * kOrders * U;
-  uint16_t *bkt = s.bkt + (v & 1) * kOrders * U;
   const int lane = t & 31, w = t >> 5;
-  uint32_t kp[2][E], a[2][E];
+  const uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
+  const uint32_t *pkey = s.key + ((v + 1) & 1) * kOrders * L.ks;
+  uint16_t *lnk = s.lnk + (v & 1) * kOrders * L.ls;
+  uint8_t *bkt = s.bkt + (v & 1) * kOrders * L.ls;
+  uint32_t k[2][E];
+  int num[2][E], prev[2][E];  // slot here; slot + 1 in the previous unit
+  uint8_t *claim[2], *pclaim[2];
+  CUCM_UNROLL
+  for (int h = 0; h < 2; h++) {
+    const int o = 2 * w + h;
+    claim[h] = s.claim + ((v & 1) * kOrders + o) * 2 * kClaim;
+    pclaim[h] = s.claim + (((v + 1) & 1) * kOrders + o) * 2 * kClaim;
+    CUCM_UNROLL
+    for (int i = 0; i < E; i++) {
+      const int j = lane + 32 * i;
+      k[h][i] = j < nvalid ? key[o * L.ks + j] : 0u;
+    }
+  }
+  // (in all of this the loads of a step stand before its stores: the compiler
+  // keeps their order, and a load behind a store waits its turn)
+  CUCM_UNROLL
+  for (int h = 0; h < 2; h++) {
+    CUCM_UNROLL
+    for (int i = 0; i < E; i++)
+      if (lane + 32 * i < nvalid) claim[h][claim_at(k[h][i], 0, kClaimLog)] = (uint8_t)(lane + 32 * i);
+  }
+  __syncwarp();
+  uint32_t open = 0;   // bits of this lane that still need a number: bit E * h + i
+  uint32_t loose = 0;  // ... whose key the previous unit's first table does not have
   CUCM_UNROLL
   for (int h = 0; h < 2; h++) {
     const int o = 2 * w + h;
     CUCM_UNROLL
     for (int i = 0; i < E; i++) {
       const int j = lane + 32 * i;
-      kp[h][i] = j < nvalid ? key[j * kOrders + o] + 1 : kNoKey;
-      a[h][i] = kp[h][i];
+      const uint32_t at = claim_at(k[h][i], 0, kClaimLog);
+      num[h][i] = claim[h][at];
+      const int p = pclaim[h][at];
+      const bool here = key[o * L.ks + num[h][i]] == k[h][i];
+      const bool there = v > 0 && pkey[o * L.ks + p] == k[h][i];
+      prev[h][i] = there ? p + 1 : 0;
+      if (j < nvalid && !here) open |= 1u << (E * h + i);
+      if (j < nvalid && !there) loose |= 1u << (E * h + i);
     }
   }
-  warp_sort<E>(a[0], lane);
-  warp_sort<E>(a[1], lane);
+  // second tables: every bit looks, the open ones claim
   CUCM_UNROLL
   for (int h = 0; h < 2; h++) {
-    uint32_t *row = s.hk + ((v & 1) * kOrders + 2 * w + h) * P;
     CUCM_UNROLL
-    for (int i = 0; i < E; i++) row[lane * E + i] = a[h][i];
+    for (int i = 0; i < E; i++)
+      if (open >> (E * h + i) & 1u) claim[h][kClaim + claim_at(k[h][i], 1, kClaimLog)] = (uint8_t)(lane + 32 * i);
   }
   __syncwarp();
   CUCM_UNROLL
   for (int h = 0; h < 2; h++) {
     const int o = 2 * w + h;
-    const uint32_t *row = s.hk + ((v & 1) * kOrders + o) * P;
-    const uint32_t *prow = s.hk + (((v + 1) & 1) * kOrders + o) * P;
+    CUCM_UNROLL
+    for (int i = 0; i < E; i++) {
+      const uint32_t bit = 1u << (E * h + i);
+      const uint32_t at = kClaim + claim_at(k[h][i], 1, kClaimLog);
+      const int n = claim[h][at], p = pclaim[h][at];
+      const bool here = key[o * L.ks + n] == k[h][i];
+      const bool there = pkey[o * L.ks + p] == k[h][i];
+      const bool take = (open & bit) && here, tie = v > 0 && (loose & bit) && there;
+      num[h][i] = take ? n : num[h][i];
+      prev[h][i] = tie ? p + 1 : prev[h][i];
+      open &= take ? ~bit : ~0u;
+      loose &= tie ? ~bit : ~0u;
+    }
+  }
+  // bits without a claim: the first one's position for all with its key
+  uint8_t *late = s.late + ((v & 1) * kOrders + 2 * w) * (L.NSLOT + 4);
+  const uint8_t *plate = s.late + (((v + 1) & 1) * kOrders + 2 * w) * (L.NSLOT + 4);
+  int nlate[2] = {0, 0};
+  if (__any_sync(0xffffffffu, open != 0)) {
+    CUCM_UNROLL
+    for (int h = 0; h < 2; h++) {
+      CUCM_UNROLL
+      for (int i = 0; i < E; i++) {
+        uint32_t m;
+        while ((m = __ballot_sync(0xffffffffu, open >> (E * h + i) & 1u)) != 0) {
+          const int src = __ffs(m) - 1;
+          const uint32_t kk = __shfl_sync(0xffffffffu, k[h][i], src);
+          const int n = src + 32 * i;
+          CUCM_UNROLL
+          for (int q = 0; q < E; q++)
+            if ((open >> (E * h + q) & 1u) && k[h][q] == kk) {
+              num[h][q] = n;
+              open &= ~(1u << (E * h + q));
+            }
+          if (lane == 0) late[h * (L.NSLOT + 4) + 4 + nlate[h]] = (uint8_t)n;
+          nlate[h]++;
+        }
+      }
+    }
+  }
+  CUCM_UNROLL
+  for (int h = 0; h < 2; h++) {
+    const int o = 2 * w + h;
+    const int np = v > 0 ? plate[h * (L.NSLOT + 4)] : 0;
+    for (int q = 0; q < np; q++) {
+      const int n = plate[h * (L.NSLOT + 4) + 4 + q];
+      const uint32_t kk = pkey[o * L.ks + n];
+      CUCM_UNROLL
+      for (int i = 0; i < E; i++)
+        if ((loose >> (E * h + i) & 1u) && k[h][i] == kk) prev[h][i] = n + 1;
+    }
+    if (lane == 0) late[h * (L.NSLOT + 4)] = (uint8_t)nlate[h];
     CUCM_UNROLL
     for (int i = 0; i < E; i++) {
       const int j = lane + 32 * i;
       if (j < nvalid) {
-        const int d = row_find<P>(row, kp[h][i]);
-        const int pd = row_find<P>(prow, kp[h][i]);
-        bkt[j * kOrders + o] = (uint16_t)d;
-        lnk[j * kOrders + o] = (uint16_t)(prow[pd] == kp[h][i] ? pd + 1 : 0);
+        bkt[o * L.ls + j] = (uint8_t)num[h][i];
+        lnk[o * L.ls + j] = (uint16_t)prev[h][i];
       }
     }
   }
@@ -306,21 +352,21 @@ __device__ __forceinline__ void walk_unit(const FastSmem &s, const FastLayout &L
                                           int n) {
   const int U = L.U, NS = L.NSLOT;
   const int o = lane & 7, r0 = lane >> 3;
-  const uint32_t *hk = s.hk + ((v & 1) * kOrders + o) * NS;
-  const uint16_t *lnk = s.lnk + (v & 1) * U * kOrders;
-  const uint16_t *bkt = s.bkt + (v & 1) * U * kOrders;
+  const uint32_t *key = s.key + ((v & 1) * kOrders + o) * L.ks;
+  const uint16_t *lnk = s.lnk + ((v & 1) * kOrders + o) * L.ls;
+  const uint8_t *bkt = s.bkt + ((v & 1) * kOrders + o) * L.ls;
   const uint8_t *fsb = s.fsw + (v & 1) * U * kOrders;
   const uint32_t *yw = s.yw + (v & 3) * (U / 32);
   uint8_t *st = s.st + (v & 1) * U * kOrders;
   uint8_t *fr = s.fr + (v & 1) * U * kOrders;
-  uint16_t *ns_cur = s.ns + ((v & 1) * kOrders + o) * NS;
-  const uint16_t *ns_prev = s.ns + (((v + 1) & 1) * kOrders + o) * NS;
+  uint8_t *ns_cur = s.ns + ((v & 1) * kOrders + o) * NS;
+  const uint8_t *ns_prev = s.ns + (((v + 1) & 1) * kOrders + o) * NS;
   uint8_t *tab = slot + table_offset(o);
   const FastTables *tb = s.tab;
   for (int q = 0; q < (n >> 3); q++) {
     const int ja = q * 8 + r0, jb = ja + 4;
     const int ia = ja * kOrders + o, ib = jb * kOrders + o;
-    const uint32_t ba = bkt[ia], bb = bkt[ib];
+    const uint32_t ba = bkt[ja], bb = bkt[jb];
     // the byte's 8 slots of this order: any two alike?
     bool clash = ba == bb;
 CUCM_UNROLL
@@ -330,39 +376,39 @@ CUCM_UNROLL
       clash |= (k != r0) && (oa == ba || ob == ba || oa == bb || ob == bb);
     }
     if (!__any_sync(0xffffffffu, clash)) {
-      const uint32_t ca = lnk[ia], cb = lnk[ib];
-      const uint32_t fa = ca ? (uint32_t)(ns_prev[ca - 1] & 0xffu) : (uint32_t)fsb[ia];
-      const uint32_t fb = cb ? (uint32_t)(ns_prev[cb - 1] & 0xffu) : (uint32_t)fsb[ib];
+      const uint32_t ca = lnk[ja], cb = lnk[jb];
+      const uint32_t fa = ca ? (uint32_t)ns_prev[ca - 1] : (uint32_t)fsb[ia];
+      const uint32_t fb = cb ? (uint32_t)ns_prev[cb - 1] : (uint32_t)fsb[ib];
       const uint32_t na = ns_cur[ba], nb = ns_cur[bb];
-      const uint32_t ka = hk[ba], kb = hk[bb];
+      const uint32_t ka = key[ja], kb = key[jb];
       const uint32_t yword = yw[q >> 2];
       const uint32_t ya = (yword >> (ja & 31)) & 1u, yb = (yword >> (jb & 31)) & 1u;
-      const uint32_t la = (na & 0x100u) ? (na & 0xffu) : fa;
-      const uint32_t lb = (nb & 0x100u) ? (nb & 0xffu) : fb;
+      const uint32_t la = na != kUntouched ? na : fa;
+      const uint32_t lb = nb != kUntouched ? nb : fb;
       const uint32_t sa = tb->nex[la][ya], sb = tb->nex[lb][yb];
-      ns_cur[ba] = (uint16_t)(0x100u | sa);
-      ns_cur[bb] = (uint16_t)(0x100u | sb);
+      ns_cur[ba] = (uint8_t)sa;
+      ns_cur[bb] = (uint8_t)sb;
       st[ia] = (uint8_t)la;
       st[ib] = (uint8_t)lb;
       fr[ia] = (uint8_t)fa;
       fr[ib] = (uint8_t)fb;
-      tab[ka - 1] = (uint8_t)sa;  // write-through; later touches overwrite it
-      tab[kb - 1] = (uint8_t)sb;
+      tab[ka] = (uint8_t)sa;  // write-through; later touches overwrite it
+      tab[kb] = (uint8_t)sb;
     } else if (lane < kOrders) {
       // bit by bit for this byte, lane = order
       for (int r = 0; r < 8; r++) {
         const int j = q * 8 + r, i = j * kOrders + lane;
-        const uint32_t b = bkt[i];
-        const uint32_t c = lnk[i];
-        const uint32_t f = c ? (uint32_t)(ns_prev[c - 1] & 0xffu) : (uint32_t)fsb[i];
+        const uint32_t b = bkt[j];
+        const uint32_t c = lnk[j];
+        const uint32_t f = c ? (uint32_t)ns_prev[c - 1] : (uint32_t)fsb[i];
         const uint32_t nc = ns_cur[b];
         const uint32_t y = (yw[j >> 5] >> (j & 31)) & 1u;
-        const uint32_t lv = (nc & 0x100u) ? (nc & 0xffu) : f;
+        const uint32_t lv = nc != kUntouched ? nc : f;
         const uint32_t ns = tb->nex[lv][y];
-        ns_cur[b] = (uint16_t)(0x100u | ns);
+        ns_cur[b] = (uint8_t)ns;
         st[i] = (uint8_t)lv;
         fr[i] = (uint8_t)f;
-        tab[hk[b] - 1] = (uint8_t)ns;
+        tab[key[j]] = (uint8_t)ns;
       }
     }
     __syncwarp();
@@ -479,50 +525,61 @@ __device__ __forceinline__ void front_mix(const FastSmem &s, const FastLayout &L
     }
   }
   front_sync();  // every weight read before any update
+  // Lane l adds its order (l + i) % 8 at step i: the bits of a warp mostly
+  // share a few rows, and the same order at a time would send all 32 adds to
+  // those rows' one word (and 4 banks).
   CUCM_UNROLL
   for (int h = 0; h < 2; h++) {
     if (has[h]) {
+      int d[kOrders];
       CUCM_UNROLL
-      for (int o = 0; o < kOrders; o++) {
-        const int d = (int)(((long long)errs[h] * smps[h][o]) >> 16);
-        atomicAdd(&s.w[cxs[h] * kOrders + o], d);
+      for (int o = 0; o < kOrders; o++) d[o] = (int)(((long long)errs[h] * smps[h][o]) >> 16);
+      CUCM_UNROLL
+      for (int k = 1; k < kOrders; k <<= 1) {
+        int e[kOrders];
+        CUCM_UNROLL
+        for (int o = 0; o < kOrders; o++) e[o] = (t & k) ? d[(o + k) & 7] : d[o];
+        CUCM_UNROLL
+        for (int o = 0; o < kOrders; o++) d[o] = e[o];
       }
+      CUCM_UNROLL
+      for (int i = 0; i < kOrders; i++) atomicAdd(&s.w[cxs[h] * kOrders + ((t + i) & 7)], d[i]);
     }
   }
 }
 
 // Front: table words holding the slot states of unit v, into registers.
-// Each thread takes entries e = t + 128 i (i < GR) of the [8][U] grid; GR is
-// 8 for units up to 128 bits and 16 up to 256.
+// Thread t takes the 8 orders of bits t and t + 128; GR is 8 for units up to
+// 128 bits and 16 up to 256.
 template <int GR>
 __device__ __forceinline__ void front_gather(const FastSmem &s, const FastLayout &L, const uint8_t *slot, int t,
                                              int v, int nvalid, uint32_t g[GR]) {
-  const int U = L.U;
-  const uint32_t *key = s.key + (v & 1) * kOrders * U;
+  const uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
   CUCM_UNROLL
   for (int i = 0; i < GR; i++) {
-    const int e = t + i * kFrontThreads;
-    if (e < kOrders * U) {
-      const int j = e >> 3, o = e & 7;
-      if (j < nvalid) {
-        const uint32_t k = key[e];
-        const uint32_t *p = reinterpret_cast<const uint32_t *>(slot + table_offset(o) + (k & ~3u));
-        g[i] = __ldcg(p);
-      }
+    const int j = t + (i >> 3) * kFrontThreads, o = i & 7;
+    if (j < nvalid) {
+      const uint32_t k = key[o * L.ks + j];
+      g[i] = __ldcg(reinterpret_cast<const uint32_t *>(slot + table_offset(o) + (k & ~3u)));
     }
   }
 }
 
 template <int GR>
-__device__ __forceinline__ void front_store_gather(const FastSmem &s, const FastLayout &L, int t, int v,
+__device__ __forceinline__ void front_store_gather(const FastSmem &s, const FastLayout &L, int t, int v, int nvalid,
                                                    const uint32_t g[GR]) {
-  const int U = L.U;
-  const uint32_t *key = s.key + (v & 1) * kOrders * U;
-  uint8_t *fsb = s.fsw + (v & 1) * kOrders * U;
+  const uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
+  uint8_t *fsb = s.fsw + (v & 1) * kOrders * L.U;
   CUCM_UNROLL
-  for (int i = 0; i < GR; i++) {
-    const int e = t + i * kFrontThreads;
-    if (e < kOrders * U) fsb[e] = (uint8_t)(g[i] >> (8 * (key[e] & 3)));
+  for (int h = 0; h < GR / 8; h++) {
+    const int j = t + h * kFrontThreads;
+    if (j < nvalid) {
+      uint32_t b[kOrders];
+      CUCM_UNROLL
+      for (int o = 0; o < kOrders; o++) b[o] = (g[8 * h + o] >> (8 * (key[o * L.ks + j] & 3))) & 0xffu;
+      *reinterpret_cast<uint2 *>(fsb + j * kOrders) =
+          make_uint2(b[0] | b[1] << 8 | b[2] << 16 | b[3] << 24, b[4] | b[5] << 8 | b[6] << 16 | b[7] << 24);
+    }
   }
 }
 
@@ -557,38 +614,44 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
   }
   for (int i = tid; i < kMixCtx * kOrders; i += blockDim.x) s.w[i] = init->w[i];
   for (int i = tid; i < 2 * U; i += blockDim.x) s.prm[i] = coder_entry(0);  // cucm_compress_v2.cu:1039-1040
-  for (int i = tid; i < 2 * kOrders * L.NSLOT; i += blockDim.x) s.hk[i] = 0;
+  for (int i = tid; i < 4 * kOrders * kClaim; i += blockDim.x) s.claim[i] = 0;  // (any position is a valid one)
 
   Coder c{0u, 0xffffffffu, 0, 0};
   uint32_t g[GR];
   uint32_t wbyte = 0;
   __syncthreads();
 
-  // Prologue: keys of units 0 and 1, links and gathers of unit 0.
+  // Prologue: keys, links and gathers of unit 0.
   if (front) {
-    for (int v = 0; v < 2 && v < nU; v++) {
-      const uint32_t b = window_load(t.in, len, U, v, ft);
-      if (ft < U / 8 + 7) s.win[ft] = (uint8_t)b;
-      front_sync();
-      front_keys(s, L, ft, v, fast_nvalid(data_bits, U, v));
-      front_sync();
-    }
+    wbyte = window_load(t.in, len, U, 0, ft);
+    if (ft < U / 8 + 7) s.win[ft] = (uint8_t)wbyte;
+    front_sync();
+    front_keys(s, L, ft, 0, fast_nvalid(data_bits, U, 0));
+    front_sync();
     front_links<GR / 2>(s, L, ft, 0, fast_nvalid(data_bits, U, 0));
     front_gather<GR>(s, L, slot, ft, 0, fast_nvalid(data_bits, U, 0), g);
-    front_store_gather<GR>(s, L, ft, 0, g);
-    if (nU > 2) wbyte = window_load(t.in, len, U, 2, ft);
+    front_store_gather<GR>(s, L, ft, 0, fast_nvalid(data_bits, U, 0), g);
+    if (nU > 1) wbyte = window_load(t.in, len, U, 1, ft);
   }
   __syncthreads();
 
   for (int tau = 0; tau < nU + 2; tau++) {
     const int um = tau - 1;
-    // gathers of unit tau+1 go out first; they land while the front works
     const int nv1 = fast_nvalid(data_bits, U, tau + 1);
-    if (front && tau + 1 < nU) front_gather<GR>(s, L, slot, ft, tau + 1, nv1, g);
     int smps[2][kOrders];
     if (warp == kWChain || front) {
       if (front && um >= 0 && um < nU) front_probs(s, L, ft, um, fast_nvalid(data_bits, U, um), smps);
       named_barrier(1, kSnapThreads);
+    }
+    // keys and gathers of unit tau+1; the gathers land while the front mixes
+    // and links
+    if (front && tau + 1 < nU) {
+      if (ft < U / 8 + 7) s.win[ft] = (uint8_t)wbyte;
+      front_sync();
+      front_keys(s, L, ft, tau + 1, nv1);
+      if (tau + 2 < nU) wbyte = window_load(t.in, len, U, tau + 2, ft);
+      front_sync();
+      front_gather<GR>(s, L, slot, ft, tau + 1, nv1, g);
     }
     if (warp == kWChain) {
       if (um >= 0 && um < nU && lane < kOrders) fast_chain(s, L, lane, um, fast_nvalid(data_bits, U, um));
@@ -601,7 +664,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
     } else if (warp == kWWalk) {
       if (tau < nU) {
         uint4 *z4 = reinterpret_cast<uint4 *>(s.ns + (tau & 1) * kOrders * L.NSLOT);
-        for (int i = lane; i < kOrders * L.NSLOT / 8; i += 32) z4[i] = make_uint4(0, 0, 0, 0);
+        for (int i = lane; i < kOrders * L.NSLOT / 16; i += 32) z4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
         __syncwarp();
         walk_unit(s, L, slot, lane, tau, fast_nvalid(data_bits, U, tau));
       }
@@ -609,13 +672,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
       if (um >= 0 && um < nU) front_mix(s, L, ft, um, fast_nvalid(data_bits, U, um), smps);
       if (tau + 1 < nU) {
         front_links<GR / 2>(s, L, ft, tau + 1, nv1);
-        if (tau + 2 < nU) {
-          if (ft < U / 8 + 7) s.win[ft] = (uint8_t)wbyte;
-          front_sync();
-          front_keys(s, L, ft, tau + 2, fast_nvalid(data_bits, U, tau + 2));
-          if (tau + 3 < nU) wbyte = window_load(t.in, len, U, tau + 3, ft);
-        }
-        front_store_gather<GR>(s, L, ft, tau + 1, g);
+        front_store_gather<GR>(s, L, ft, tau + 1, nv1, g);
       }
     }
     __syncthreads();
