@@ -5,9 +5,8 @@
 // The reference runs five launches per unit and a host round trip between
 // them (cucm_compress_v2.cu:1067-1090).  Here one CTA of 7 warps codes a
 // chunk, each warp owning one stage, all stages of consecutive units
-// overlapped ("tick" t).  The numbers below are roles; compress_fast_one
-// gives them to physical warps so that the chain warp has a scheduler to
-// itself:
+// overlapped ("tick" t).  The numbers below are roles (kRolesAlone and
+// kRolesPaired give them to physical warps):
 //
 //   front warps (3..6, 128 threads)
 //     * keys of unit t+1 for all 8 orders (one FNV pass per bit,
@@ -27,10 +26,10 @@
 //     sees (live), the state each prediction saw (frozen = unit-start value),
 //     the next state, written through to the slot table.  It only depends on
 //     the bits, never on the probabilities, so it runs a unit ahead of the
-//     chain.
+//     chain, and groups the unit's updates by state for it.
 //   chain warp (0, lane = order): the StateMap probability updates of unit
-//     t-1 in bit order (cucm_compress_v2.cu:592-601); the adaptation rate is
-//     carried next to each probability.
+//     t-1, state by state, each state's in bit order
+//     (cucm_compress_v2.cu:592-601).
 //   coder warp (1): the binary arithmetic coder for unit t-2.
 //
 // After the last data unit the coder keeps coding the stale unit buffer up
@@ -44,6 +43,14 @@ constexpr int kFrontThreads = 128;
 constexpr int kSnapThreads = 32 + kFrontThreads;  // chain + front warps (barrier 1)
 constexpr int kWinBytes = kFastMaxUnit / 8 + 8;    // input window of a unit (+7 history bytes)
 
+// Role of each of a CTA's warps, 4 bits a warp.  Warp i issues from the SM's
+// scheduler i % 4.  Alone on an SM, each serial role shares a scheduler with
+// front warps only; where two CTAs share an SM, the chain keeps one for itself
+// and coder and walker share one.  Each the other way round: 1 MiB at 64 KiB
+// chunks (16 CTAs) 22.1 -> 23.7 ms, 128 MiB at 512 KiB chunks (two CTAs an SM)
+// 357 -> 364 ms.
+constexpr uint32_t kRolesAlone = 0x6540213u, kRolesPaired = 0x6250413u;
+
 constexpr int kFastStageMin = 2048;
 
 // A compress CTA keeps the whole of the tables in shared memory (reading
@@ -51,14 +58,20 @@ constexpr int kFastStageMin = 2048;
 // slower: the lookups are on the front warps' critical path).
 typedef Tables FastTables;
 
+// Row padding of the walker's [order][...] arrays: 16 bytes, so that the 8
+// orders' rows start in different banks.
+constexpr int kStatePad = 16, kSortPad = 8;
+constexpr int kRecRow = 257;   // 256 states: the rows start in different banks, bits of one order spread over all
+constexpr int kChainRow = 37;  // 32 steps and 4 of read-ahead; odd, so that the rows start in different banks
+
 constexpr uint32_t kUntouched = 0xffu;  // no state: the largest is 252
 constexpr int kClaimLog = 9, kClaim = 1 << kClaimLog;  // places of a claim table
 
 struct FastLayout {
   int U, NSLOT, stage;
   int ks, ls;   // row lengths of key and of lnk / bkt
-  size_t off_tab, off_rec, off_w, off_claim, off_late, off_ns, off_key, off_lnk, off_bkt, off_fsw, off_st, off_fr,
-      off_yw, off_c1, off_prm, off_win, off_stage, total;
+  size_t off_tab, off_rec, off_w, off_claim, off_late, off_ns, off_key, off_lnk, off_bkt, off_fsw, off_st, off_srt, off_step,
+      off_fr, off_yw, off_c1, off_prm, off_win, off_stage, total;
 };
 
 __host__ __device__ inline FastLayout make_fast_layout(int U) {
@@ -77,7 +90,7 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
     return at;
   };
   L.off_tab = take(sizeof(FastTables));
-  L.off_rec = take(sizeof(uint64_t) * kOrders * 256);
+  L.off_rec = take(sizeof(uint32_t) * kOrders * kRecRow);
   L.off_w = take(sizeof(int32_t) * kMixCtx * kOrders);
   L.off_claim = take((size_t)2 * kOrders * 2 * kClaim);   // claim tables [unit parity][order][round]
   L.off_late = take((size_t)2 * kOrders * (NS + 4));       // slots claimed after the rounds [unit parity][order]
@@ -86,7 +99,9 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
   L.off_lnk = take(sizeof(uint16_t) * 2 * kOrders * L.ls); // slot + 1 in the previous unit, or 0 [unit parity][order][bit]
   L.off_bkt = take((size_t)2 * kOrders * L.ls);            // slot in this unit
   L.off_fsw = take((size_t)2 * kOrders * U);               // gathered slot states
-  L.off_st = take((size_t)2 * kOrders * U + 4 * kOrders);  // live state (+ the chain's read-ahead)
+  L.off_st = take((size_t)kOrders * (U + kStatePad));      // live state [order][bit]
+  L.off_srt = take(sizeof(uint16_t) * 2 * kOrders * (U + kSortPad));  // updates grouped by state [unit parity][order]
+  L.off_step = take((size_t)16 * kOrders * kChainRow);     // operands of 32 updates [order]
   L.off_fr = take((size_t)2 * U * kOrders);                // frozen state
   L.off_yw = take(sizeof(uint32_t) * 4 * (U / 32));        // bits, by unit mod 4
   L.off_c1 = take((size_t)4 * (U / 8));                    // previous byte per byte, by unit mod 4
@@ -97,9 +112,11 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
   return L;
 }
 
+struct ChainStep;
+
 struct FastSmem {
   FastTables *tab;
-  uint64_t *rec;     // [256][8]  statep | dt[count] << 32 | dt[count + 1] << 48
+  uint32_t *rec;     // [8][kRecRow]  statep
   int32_t *w;        // [80*8]
   uint8_t *claim;    // [2][8][2][kClaim]
   uint8_t *late;     // [2][8][NSLOT + 4]: count, slots
@@ -108,7 +125,9 @@ struct FastSmem {
   uint16_t *lnk;     // [2][8][ls]
   uint8_t *bkt;      // [2][8][ls]
   uint8_t *fsw;      // [2][U][8]
-  uint8_t *st;       // [2][U][8]
+  uint8_t *st;       // [8][U + kStatePad]
+  uint16_t *srt;     // [2][8][U + kSortPad]
+  ChainStep *step;    // [8][kChainRow]
   uint8_t *fr;       // [2][U][8]
   uint32_t *yw;      // [4][U/32]
   uint8_t *c1;       // [4][U/8]
@@ -120,7 +139,7 @@ struct FastSmem {
 __device__ inline FastSmem carve_fast(uint8_t *b, const FastLayout &L) {
   FastSmem s;
   s.tab = reinterpret_cast<FastTables *>(b + L.off_tab);
-  s.rec = reinterpret_cast<uint64_t *>(b + L.off_rec);
+  s.rec = reinterpret_cast<uint32_t *>(b + L.off_rec);
   s.w = reinterpret_cast<int32_t *>(b + L.off_w);
   s.claim = b + L.off_claim;
   s.late = b + L.off_late;
@@ -130,6 +149,8 @@ __device__ inline FastSmem carve_fast(uint8_t *b, const FastLayout &L) {
   s.bkt = b + L.off_bkt;
   s.fsw = b + L.off_fsw;
   s.st = b + L.off_st;
+  s.srt = reinterpret_cast<uint16_t *>(b + L.off_srt);
+  s.step = reinterpret_cast<ChainStep *>(b + L.off_step);
   s.fr = b + L.off_fr;
   s.yw = reinterpret_cast<uint32_t *>(b + L.off_yw);
   s.c1 = b + L.off_c1;
@@ -159,10 +180,14 @@ __device__ __forceinline__ uint32_t window_load(const uint8_t *in, uint64_t len,
   return (t < U / 8 + 7 && i >= 0 && (uint64_t)i < len) ? (uint32_t)__ldg(in + i) : 0u;
 }
 
+__device__ __forceinline__ uint32_t *keys_of(const FastSmem &s, const FastLayout &L, int v) {
+  return s.key + (v & 1) * kOrders * L.ks;
+}
+
 // Front: keys, bits and previous bytes of unit v from the staged window.
 __device__ __forceinline__ void front_keys(const FastSmem &s, const FastLayout &L, int t, int v, int nvalid) {
   const int U = L.U;
-  uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
+  uint32_t *key = keys_of(s, L, v);
   uint32_t *yw = s.yw + (v & 3) * (U / 32);
   uint8_t *c1 = s.c1 + (v & 3) * (U / 8);
   for (int j0 = 0; j0 < U; j0 += kFrontThreads) {
@@ -219,8 +244,8 @@ __device__ __forceinline__ uint32_t claim_at(uint32_t key, int round, int logn) 
 template <int E>
 __device__ __forceinline__ void front_links(const FastSmem &s, const FastLayout &L, int t, int v, int nvalid) {
   const int lane = t & 31, w = t >> 5;
-  const uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
-  const uint32_t *pkey = s.key + ((v + 1) & 1) * kOrders * L.ks;
+  const uint32_t *key = keys_of(s, L, v);
+  const uint32_t *pkey = keys_of(s, L, v + 1);
   uint16_t *lnk = s.lnk + (v & 1) * kOrders * L.ls;
   uint8_t *bkt = s.bkt + (v & 1) * kOrders * L.ls;
   uint32_t k[2][E];
@@ -338,138 +363,253 @@ __device__ __forceinline__ void front_links(const FastSmem &s, const FastLayout 
   }
 }
 
-// Walker: bit-history updates of unit v in bit order, a byte per step.  A
-// slot recurs at most once per byte except when two keys of one order
-// collide in the 25-bit hash, so the 64 updates of a byte (lane: order
-// lane & 7, bits lane >> 3 and (lane >> 3) + 4) are independent and run
-// together; a byte with a collision is walked bit by bit instead.  Per
-// update: the state it sees (live: an earlier touch in this unit, else the
-// frozen unit-start state -- from the previous unit's table when linked),
-// the next state, written through to the slot table.  It only depends on
-// the bits, never on the probabilities, so it runs a unit ahead of the
-// chain.
+// Walker: bit-history updates of unit v in bit order, a byte per step.  The 8
+// keys of a byte and an order are never alike: the bits share the previous
+// bytes and differ in the partial byte, and both steps of the hash, the XOR
+// with a byte and the product with an odd number, are one-to-one on its low 25
+// bits.  So the 64 updates of a byte (lane: order lane & 7, bits lane >> 3 and
+// (lane >> 3) + 4) are independent and run together.  Per update: the state it
+// sees (live: an earlier touch in this unit, else the frozen unit-start state
+// -- from the previous unit's table when linked), the next state, written
+// through to the slot table.  It only depends on the bits, never on the
+// probabilities, so it runs a unit ahead of the chain.  All that a step reads
+// but its slots' live states is read a step ahead, so a step waits for two
+// shared-memory loads one after the other, the live state and its successor.
+struct WalkByte {
+  uint32_t b[2], k[2], f[2], y[2];  // slot, key, frozen state, bit
+};
+
 __device__ __forceinline__ void walk_unit(const FastSmem &s, const FastLayout &L, uint8_t *slot, int lane, int v,
                                           int n) {
   const int U = L.U, NS = L.NSLOT;
   const int o = lane & 7, r0 = lane >> 3;
-  const uint32_t *key = s.key + ((v & 1) * kOrders + o) * L.ks;
+  const uint32_t *key = keys_of(s, L, v) + o * L.ks;
   const uint16_t *lnk = s.lnk + ((v & 1) * kOrders + o) * L.ls;
   const uint8_t *bkt = s.bkt + ((v & 1) * kOrders + o) * L.ls;
-  const uint8_t *fsb = s.fsw + (v & 1) * U * kOrders;
+  const uint8_t *fsb = s.fsw + (v & 1) * U * kOrders + o;
   const uint32_t *yw = s.yw + (v & 3) * (U / 32);
-  uint8_t *st = s.st + (v & 1) * U * kOrders;
-  uint8_t *fr = s.fr + (v & 1) * U * kOrders;
+  uint8_t *st = s.st + o * (U + kStatePad);
+  uint8_t *fr = s.fr + (v & 1) * U * kOrders + o;
   uint8_t *ns_cur = s.ns + ((v & 1) * kOrders + o) * NS;
   const uint8_t *ns_prev = s.ns + (((v + 1) & 1) * kOrders + o) * NS;
   uint8_t *tab = slot + table_offset(o);
   const FastTables *tb = s.tab;
-  for (int q = 0; q < (n >> 3); q++) {
-    const int ja = q * 8 + r0, jb = ja + 4;
-    const int ia = ja * kOrders + o, ib = jb * kOrders + o;
-    const uint32_t ba = bkt[ja], bb = bkt[jb];
-    // the byte's 8 slots of this order: any two alike?
-    bool clash = ba == bb;
+  auto ahead = [&](int j, WalkByte &w) {
+    const uint32_t yword = yw[j >> 5];
 CUCM_UNROLL
-    for (int k = 0; k < 4; k++) {
-      const uint32_t oa = __shfl_sync(0xffffffffu, ba, k * 8 + o);
-      const uint32_t ob = __shfl_sync(0xffffffffu, bb, k * 8 + o);
-      clash |= (k != r0) && (oa == ba || ob == ba || oa == bb || ob == bb);
+    for (int h = 0; h < 2; h++) {
+      const int jj = j + r0 + 4 * h;
+      w.b[h] = bkt[jj];
+      w.k[h] = key[jj];
+      const uint32_t c = lnk[jj];
+      const uint32_t g = fsb[jj * kOrders];
+      w.f[h] = c ? (uint32_t)ns_prev[c - 1] : g;
+      w.y[h] = (yword >> (jj & 31)) & 1u;
     }
-    if (!__any_sync(0xffffffffu, clash)) {
-      const uint32_t ca = lnk[ja], cb = lnk[jb];
-      const uint32_t fa = ca ? (uint32_t)ns_prev[ca - 1] : (uint32_t)fsb[ia];
-      const uint32_t fb = cb ? (uint32_t)ns_prev[cb - 1] : (uint32_t)fsb[ib];
-      const uint32_t na = ns_cur[ba], nb = ns_cur[bb];
-      const uint32_t ka = key[ja], kb = key[jb];
-      const uint32_t yword = yw[q >> 2];
-      const uint32_t ya = (yword >> (ja & 31)) & 1u, yb = (yword >> (jb & 31)) & 1u;
-      const uint32_t la = na != kUntouched ? na : fa;
-      const uint32_t lb = nb != kUntouched ? nb : fb;
-      const uint32_t sa = tb->nex[la][ya], sb = tb->nex[lb][yb];
-      ns_cur[ba] = (uint8_t)sa;
-      ns_cur[bb] = (uint8_t)sb;
-      st[ia] = (uint8_t)la;
-      st[ib] = (uint8_t)lb;
-      fr[ia] = (uint8_t)fa;
-      fr[ib] = (uint8_t)fb;
-      tab[ka] = (uint8_t)sa;  // write-through; later touches overwrite it
-      tab[kb] = (uint8_t)sb;
-    } else if (lane < kOrders) {
-      // bit by bit for this byte, lane = order
-      for (int r = 0; r < 8; r++) {
-        const int j = q * 8 + r, i = j * kOrders + lane;
-        const uint32_t b = bkt[j];
-        const uint32_t c = lnk[j];
-        const uint32_t f = c ? (uint32_t)ns_prev[c - 1] : (uint32_t)fsb[i];
-        const uint32_t nc = ns_cur[b];
-        const uint32_t y = (yw[j >> 5] >> (j & 31)) & 1u;
-        const uint32_t lv = nc != kUntouched ? nc : f;
-        const uint32_t ns = tb->nex[lv][y];
-        ns_cur[b] = (uint8_t)ns;
-        st[i] = (uint8_t)lv;
-        fr[i] = (uint8_t)f;
-        tab[key[j]] = (uint8_t)ns;
-      }
-    }
+  };
+  WalkByte w;
+  ahead(0, w);
+  for (int j = 0; j < n; j += 8) {
+    const WalkByte c = w;
+    const uint32_t n0 = ns_cur[c.b[0]], n1 = ns_cur[c.b[1]];
+    if (j + 8 < n) ahead(j + 8, w);
+    const uint32_t l0 = n0 != kUntouched ? n0 : c.f[0];
+    const uint32_t l1 = n1 != kUntouched ? n1 : c.f[1];
+    const uint32_t s0 = tb->nex[l0][c.y[0]], s1 = tb->nex[l1][c.y[1]];
+    ns_cur[c.b[0]] = (uint8_t)s0;
+    ns_cur[c.b[1]] = (uint8_t)s1;
     __syncwarp();
+    const int j0 = j + r0, j1 = j0 + 4;
+    st[j0] = (uint8_t)l0;
+    st[j1] = (uint8_t)l1;
+    fr[j0 * kOrders] = (uint8_t)c.f[0];
+    fr[j1 * kOrders] = (uint8_t)c.f[1];
+    tab[c.k[0]] = (uint8_t)s0;  // write-through; later touches overwrite it
+    tab[c.k[1]] = (uint8_t)s1;
+  }
+  __syncwarp();
+}
+
+// Walker: groups unit v's StateMap updates by state for the chain warp.  Per
+// order and 128 bits, the updates (state << 8 | bit << 1 | y) in ascending
+// order: states apart, the updates of one state in bit order.  Lane = (order
+// lane & 7, quarter lane >> 3) sorts its 32 bits, two 16-bit keys to a
+// register, then the quarters are merged across lanes.  Updates of different
+// states of an order never meet, so this is all the order the chain needs.
+__device__ __forceinline__ void sort_ce(uint32_t &a, uint32_t &b) {
+  const uint32_t m = __vminu2(a, b);
+  b = __vmaxu2(a, b);
+  a = m;
+}
+__device__ __forceinline__ uint32_t swap_halves(uint32_t a) { return __byte_perm(a, 0, 0x1032); }
+
+// 32 keys of a lane, key k in the low half and key 16 + k in the high half of
+// r[k]: the last steps of a bitonic merge, distances 16, 8, 4, 2, 1.
+__device__ __forceinline__ void sort_merge32(uint32_t (&r)[16], bool halves) {
+  if (halves) {
+CUCM_UNROLL
+    for (int k = 0; k < 16; k++) {
+      const uint32_t w = swap_halves(r[k]);
+      r[k] = __byte_perm(__vminu2(r[k], w), __vmaxu2(r[k], w), 0x5410);
+    }
+  }
+CUCM_UNROLL
+  for (int d = 8; d > 0; d >>= 1)
+CUCM_UNROLL
+    for (int k = 0; k < 16; k++)
+      if ((k & d) == 0) sort_ce(r[k], r[k | d]);
+}
+
+// This lane's keys against those of lane ^ lanes in reverse (a first merge
+// step) or position by position (a later one): the smaller or larger ones.
+__device__ __forceinline__ void sort_cross(uint32_t (&r)[16], int lanes, bool reverse, bool low) {
+  uint32_t w[16];
+CUCM_UNROLL
+  for (int k = 0; k < 16; k++) w[k] = __shfl_xor_sync(0xffffffffu, r[k], lanes);
+CUCM_UNROLL
+  for (int k = 0; k < 16; k++) {
+    const uint32_t x = reverse ? swap_halves(w[15 - k]) : w[k];
+    r[k] = low ? __vminu2(r[k], x) : __vmaxu2(r[k], x);
   }
 }
 
-// Chain (lane = order): StateMap probability updates of unit v in bit order.
-// A record is statep | dt[c] << 32 | dt[c+1] << 48 for the state's count c;
-// the count only ever grows by one per update, so a run of updates of one
-// state needs each table value two steps after it is requested.  A step's
-// record is loaded two steps ahead; the two results not yet stored when it
-// was loaded (the previous step's, stored one step late, and the current
-// one) are forwarded from registers, so no shared-memory round trip sits on
-// the step-to-step chain.  The bits come 32 to a word; the state three
-// steps ahead is read unconditionally (the live-state array has room past
-// its end for it).
-__device__ __forceinline__ void fast_chain(const FastSmem &s, const FastLayout &L, int o, int v, int n) {
+__device__ __forceinline__ void walk_sort(const FastSmem &s, const FastLayout &L, int lane, int v, int n) {
   const int U = L.U;
-  const uint8_t *sta = s.st + (v & 1) * U * kOrders + o;
+  const int o = lane & 7, q = lane >> 3;
   const uint32_t *yw = s.yw + (v & 3) * (U / 32);
-  uint64_t *rec = s.rec + o;  // rec[state * 8 + order]
-  const uint16_t *dt = s.tab->dt;
-  int st = sta[0];
-  int st1 = n > 1 ? sta[kOrders] : 0;
-  int st2 = n > 2 ? sta[2 * kOrders] : 0;
-  const uint64_t r0 = rec[st * kOrders];
-  uint64_t nraw = rec[st1 * kOrders];
-  uint32_t val = (uint32_t)r0, d = (uint32_t)(r0 >> 32) & 0xffffu, dn = (uint32_t)(r0 >> 48);
-  int pst = st;
-  uint32_t pv = val, pd = d, pdn = dn;
-  for (int j0 = 0; j0 < n; j0 += 32) {
-    uint32_t ywd = yw[j0 >> 5];
-    const int je = j0 + 32 < n ? j0 + 32 : n;
-    for (int j = j0; j < je; j++) {
-      rec[pst * kOrders] = (uint64_t)pv | ((uint64_t)pd << 32) | ((uint64_t)pdn << 48);
-      const uint64_t r2 = rec[st2 * kOrders];
-      const int st3 = sta[(j + 3) * kOrders];
-      const uint32_t y = ywd & 1u;
-      ywd >>= 1;
-      const uint32_t cnt = val & 1023u;
-      const uint32_t dnn = dt[cnt < 1021u ? cnt + 2 : 1023u];
-      const int32_t err = (int32_t)((y << 22) - (val >> 10));
-      const uint32_t v2 = val + (((uint32_t)(err >> 3) * d) & 0xfffffc00u) + (cnt < 1023u ? 1u : 0u);
-      const bool f0 = st1 == st, f1 = st1 == pst;
-      const uint32_t nv = f0 ? v2 : f1 ? pv : (uint32_t)nraw;
-      const uint32_t nd = f0 ? dn : f1 ? pd : (uint32_t)(nraw >> 32) & 0xffffu;
-      const uint32_t ndn = f0 ? dnn : f1 ? pdn : (uint32_t)(nraw >> 48);
-      pst = st;
-      pv = v2;
-      pd = dn;
-      pdn = dnn;
-      val = nv;
-      d = nd;
-      dn = ndn;
-      nraw = r2;
-      st = st1;
-      st1 = st2;
-      st2 = st3;
+  for (int j0 = 0; j0 < n; j0 += 128) {
+    const int jq = j0 + 32 * q;  // first bit of this lane
+    const int have = n - jq;     // a multiple of 8
+    uint32_t r[16];
+    if (have > 0) {
+      const uint32_t y = yw[jq >> 5];
+      const uint4 *src = reinterpret_cast<const uint4 *>(s.st + o * (U + kStatePad) + jq);
+      const uint4 a = src[0], b = src[1];
+      const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+CUCM_UNROLL
+      for (int k = 0; k < 16; k++) {  // bits 2k and 2k + 1
+        const uint32_t st = __byte_perm(w[k >> 1], 0, k & 1 ? 0x3424 : 0x1404);
+        const uint32_t bits = (uint32_t)(32 * q) * 0x20002u + (uint32_t)(4 * k) + ((uint32_t)(4 * k + 2) << 16);
+        r[k] = st | bits | ((y >> (2 * k)) & 1u) | (((y >> (2 * k + 1)) & 1u) << 16);
+        if (2 * k >= have) r[k] = 0xffffffffu;
+      }
+    } else {
+CUCM_UNROLL
+      for (int k = 0; k < 16; k++) r[k] = 0xffffffffu;
+    }
+    // the low and the high halves, 16 keys each (Batcher's merge exchange)
+CUCM_UNROLL
+    for (int p = 1; p < 16; p *= 2)
+CUCM_UNROLL
+      for (int k = p; k >= 1; k /= 2)
+CUCM_UNROLL
+        for (int i = 0; i < 16; i++)
+          if (i + k < 16 && i >= k % p && (i - k % p) % (2 * k) < k && i / (2 * p) == (i + k) / (2 * p))
+            sort_ce(r[i], r[i + k]);
+    // the two halves of a lane
+CUCM_UNROLL
+    for (int k = 0; k < 8; k++) {
+      const uint32_t w = swap_halves(r[15 - k]);
+      const uint32_t m = __vminu2(r[k], w), x = __vmaxu2(r[k], w);
+      r[k] = __byte_perm(m, x, 0x5410);
+      r[15 - k] = __byte_perm(m, x, 0x7632);
+    }
+    sort_merge32(r, false);
+    if (n - j0 > 32) {
+      sort_cross(r, 8, true, (q & 1) == 0);
+      sort_merge32(r, true);
+    }
+    if (n - j0 > 64) {
+      sort_cross(r, 24, true, q < 2);
+      sort_cross(r, 8, false, (q & 1) == 0);
+      sort_merge32(r, true);
+    }
+    if (have > 0) {
+      uint4 *dst = reinterpret_cast<uint4 *>(s.srt + ((v & 1) * kOrders + o) * (U + kSortPad) + jq);
+CUCM_UNROLL
+      for (int h = 0; h < 4; h++) {
+        const uint32_t sel = h < 2 ? 0x5410 : 0x7632;
+        const int k = 8 * (h & 1);
+        dst[h] = make_uint4(__byte_perm(r[k], r[k + 1], sel), __byte_perm(r[k + 2], r[k + 3], sel),
+                            __byte_perm(r[k + 4], r[k + 5], sel), __byte_perm(r[k + 6], r[k + 7], sel));
+      }
     }
   }
-  rec[pst * kOrders] = (uint64_t)pv | ((uint64_t)pd << 32) | ((uint64_t)pdn << 48);
+}
+
+// Chain (lane = order): StateMap probability updates of unit v
+// (cucm_compress_v2.cu:592-601), state by state in the order walk_sort left
+// them.  The updates of one state follow one another with its probability in
+// a register; everything else -- the probability a state starts from, its
+// count, which only ever grows by one per update, and so each update's
+// adaptation rate -- is known ahead, and read a block of 8 updates early.
+// Seven dependent operations a step; the ~35 instructions of a step bound it
+// (80 cycles, against 110 for the bits in order with every record stored and
+// the next one forwarded or loaded).  Working the operands out with all 32
+// lanes first, for 8 lanes to run through, measured the same (units of 128
+// bits) or 14 % slower (256).
+struct ChainBlock {
+  uint32_t at[8];   // record index | 0x8000 where a state begins
+  uint32_t v[8];    // probability the state begins with
+  uint32_t d[8];    // -rate
+  uint32_t k[8];    // (y << 19) * rate
+  uint32_t inc;     // bit i: the count still grows
+};
+
+__device__ __forceinline__ void chain_block(ChainBlock &b, const uint32_t *rec, const uint16_t *dt, const uint4 &e4,
+                                            uint32_t &prev, uint32_t &cnt) {
+  const uint32_t w[4] = {e4.x, e4.y, e4.z, e4.w};
+  uint32_t e[8];
+  b.inc = 0;
+CUCM_UNROLL
+  for (int i = 0; i < 8; i++) {
+    e[i] = i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu;
+    b.at[i] = e[i] >> 8;
+    b.v[i] = rec[b.at[i]];
+  }
+CUCM_UNROLL
+  for (int i = 0; i < 8; i++) {
+    const bool first = (e[i] ^ prev) >= 256u;
+    prev = e[i];
+    cnt = first ? b.v[i] & 1023u : min(cnt + 1, 1023u);
+    if (first) b.at[i] |= 0x8000u;
+    const uint32_t r = dt[cnt];
+    b.d[i] = 0u - r;
+    b.k[i] = (e[i] & 1u) ? r << 19 : 0u;
+    if (cnt < 1023u) b.inc |= 1u << i;
+  }
+}
+
+__device__ __forceinline__ void chain_run(const ChainBlock &b, uint32_t *rec, uint32_t &val) {
+CUCM_UNROLL
+  for (int i = 0; i < 8; i++) {
+    const uint32_t x = (b.at[i] & 0x8000u) ? b.v[i] : val;
+    // (err >> 3) * rate with err = (y << 22) - (x >> 10)
+    const uint32_t t = ((x >> 10) + 7u) >> 3;
+    val = x + (((b.k[i] + t * b.d[i]) & 0xfffffc00u) | ((b.inc >> i) & 1u));
+    rec[b.at[i] & 0x7fffu] = val;
+  }
+}
+
+__device__ __forceinline__ void fast_chain(const FastSmem &s, const FastLayout &L, int o, int v, int n) {
+  uint32_t *rec = s.rec + o * kRecRow;
+  const uint16_t *dt = s.tab->dt;
+  const uint4 *src = reinterpret_cast<const uint4 *>(s.srt + ((v & 1) * kOrders + o) * (L.U + kSortPad));
+  for (int j0 = 0; j0 < n; j0 += 128) {
+    const int nb = (n - j0 < 128 ? n - j0 : 128) >> 3;  // blocks (n is a multiple of 8)
+    uint32_t prev = 0x10000u, cnt = 0, val = 0;
+    ChainBlock cur, nxt;
+    chain_block(cur, rec, dt, src[0], prev, cnt);
+    for (int i = 1; i < nb; i++) {
+      // only states that begin in the next block use what is read here, and
+      // no earlier block has touched those
+      chain_block(nxt, rec, dt, src[i], prev, cnt);
+      chain_run(cur, rec, val);
+      cur = nxt;
+    }
+    chain_run(cur, rec, val);
+    src += 16;
+  }
 }
 
 // Front: stretched probabilities of unit v's bits (thread t: bits t and
@@ -487,7 +627,7 @@ __device__ __forceinline__ void front_probs(const FastSmem &s, const FastLayout 
       CUCM_UNROLL
       for (int o = 0; o < kOrders; o++) {
         const uint32_t stt = (uint32_t)(f8 >> (8 * o)) & 0xffu;
-        smps[h][o] = s.tab->stretch[reinterpret_cast<const uint32_t *>(s.rec)[2 * (stt * kOrders + o)] >> 20];
+        smps[h][o] = s.tab->stretch[s.rec[o * kRecRow + stt] >> 20];
       }
     }
   }
@@ -554,7 +694,7 @@ __device__ __forceinline__ void front_mix(const FastSmem &s, const FastLayout &L
 template <int GR>
 __device__ __forceinline__ void front_gather(const FastSmem &s, const FastLayout &L, const uint8_t *slot, int t,
                                              int v, int nvalid, uint32_t g[GR]) {
-  const uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
+  const uint32_t *key = keys_of(s, L, v);
   CUCM_UNROLL
   for (int i = 0; i < GR; i++) {
     const int j = t + (i >> 3) * kFrontThreads, o = i & 7;
@@ -568,7 +708,7 @@ __device__ __forceinline__ void front_gather(const FastSmem &s, const FastLayout
 template <int GR>
 __device__ __forceinline__ void front_store_gather(const FastSmem &s, const FastLayout &L, int t, int v, int nvalid,
                                                    const uint32_t g[GR]) {
-  const uint32_t *key = s.key + (v & 1) * kOrders * L.ks;
+  const uint32_t *key = keys_of(s, L, v);
   uint8_t *fsb = s.fsw + (v & 1) * kOrders * L.U;
   CUCM_UNROLL
   for (int h = 0; h < GR / 8; h++) {
@@ -587,14 +727,11 @@ constexpr uint64_t kTailOffloadBits = 4096;  // shorter stale tails are coded in
 
 template <int GR>
 __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastSmem &s, const FastLayout &L,
-                                  const ModelInit *init, uint32_t *status, TailTask *tails, uint32_t *tail_count) {
+                                  const ModelInit *init, uint32_t *status, TailTask *tails, uint32_t *tail_count,
+                                  uint32_t roles) {
   const int tid = threadIdx.x;
   const int pw = tid >> 5, lane = tid & 31;
-  // Role of each warp.  A CTA's warp i issues from the SM's scheduler i % 4,
-  // so warp 3 (alone on its scheduler) takes the chain, the slowest role;
-  // the coder shares a scheduler with the walker, the front warps pair up
-  // (measured 795 -> 753 ms per 256 MiB launch against roles in warp order).
-  const int warp = (int)((0x6250413u >> (4 * pw)) & 15u);
+  const int warp = (int)((roles >> (4 * pw)) & 15u);
   const int U = L.U;
   const uint64_t len = t.in_len < t.cs ? t.in_len : t.cs;
   const uint64_t total_bits = 8ull * t.cs;
@@ -607,11 +744,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
     return b >= total_bits ? 0 : (int)(total_bits - b < (uint64_t)U ? total_bits - b : (uint64_t)U);
   };
 
-  for (int i = tid; i < kOrders * 256; i += blockDim.x) {
-    const uint32_t v = init->statep[i & 7][i >> 3];  // rec[state * 8 + order]
-    const uint32_t c = v & 1023u;
-    s.rec[i] = (uint64_t)v | ((uint64_t)s.tab->dt[c] << 32) | ((uint64_t)s.tab->dt[c < 1023u ? c + 1 : 1023u] << 48);
-  }
+  for (int i = tid; i < kOrders * 256; i += blockDim.x) s.rec[(i >> 8) * kRecRow + (i & 255)] = init->statep[i >> 8][i & 255];
   for (int i = tid; i < kMixCtx * kOrders; i += blockDim.x) s.w[i] = init->w[i];
   for (int i = tid; i < 2 * U; i += blockDim.x) s.prm[i] = coder_entry(0);  // cucm_compress_v2.cu:1039-1040
   for (int i = tid; i < 4 * kOrders * kClaim; i += blockDim.x) s.claim[i] = 0;  // (any position is a valid one)
@@ -627,11 +760,11 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
     if (ft < U / 8 + 7) s.win[ft] = (uint8_t)wbyte;
     front_sync();
     front_keys(s, L, ft, 0, fast_nvalid(data_bits, U, 0));
+    if (nU > 1) wbyte = window_load(t.in, len, U, 1, ft);
     front_sync();
     front_links<GR / 2>(s, L, ft, 0, fast_nvalid(data_bits, U, 0));
     front_gather<GR>(s, L, slot, ft, 0, fast_nvalid(data_bits, U, 0), g);
     front_store_gather<GR>(s, L, ft, 0, fast_nvalid(data_bits, U, 0), g);
-    if (nU > 1) wbyte = window_load(t.in, len, U, 1, ft);
   }
   __syncthreads();
 
@@ -644,7 +777,8 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
       named_barrier(1, kSnapThreads);
     }
     // keys and gathers of unit tau+1; the gathers land while the front mixes
-    // and links
+    // and links (keys a tick earlier, so that the gathers can go out first:
+    // within 2 % either way, and a third unit's keys to keep)
     if (front && tau + 1 < nU) {
       if (ft < U / 8 + 7) s.win[ft] = (uint8_t)wbyte;
       front_sync();
@@ -667,6 +801,7 @@ __device__ void compress_fast_one(const ChunkTask &t, uint8_t *slot, const FastS
         for (int i = lane; i < kOrders * L.NSLOT / 16; i += 32) z4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
         __syncwarp();
         walk_unit(s, L, slot, lane, tau, fast_nvalid(data_bits, U, tau));
+        walk_sort(s, L, lane, tau, fast_nvalid(data_bits, U, tau));
       }
     } else {
       if (um >= 0 && um < nU) front_mix(s, L, ft, um, fast_nvalid(data_bits, U, um), smps);
@@ -725,7 +860,7 @@ template <int GR>
 __device__ __forceinline__ void compress_fast_loop(const ChunkTask *tasks, uint32_t ntasks, uint8_t *slots,
                                                    const uint8_t *init_tables, const ModelInit *init,
                                                    uint32_t *queue, uint32_t *status, int unit, TailTask *tails,
-                                                   uint32_t *tail_count) {
+                                                   uint32_t *tail_count, uint32_t roles) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const FastLayout L = make_fast_layout(unit);
   const FastSmem s = carve_fast(smem_raw, L);
@@ -752,7 +887,7 @@ __device__ __forceinline__ void compress_fast_loop(const ChunkTask *tasks, uint3
       __syncthreads();
     }
     fresh = false;
-    compress_fast_one<GR>(t, slot, s, L, init, status, tails, tail_count);
+    compress_fast_one<GR>(t, slot, s, L, init, status, tails, tail_count, roles);
   }
 }
 
@@ -761,16 +896,16 @@ __device__ __forceinline__ void compress_fast_loop(const ChunkTask *tasks, uint3
 __global__ void __launch_bounds__(kFastThreads, 2)
     compress_fast_kernel(const ChunkTask *tasks, uint32_t ntasks, uint8_t *slots, const uint8_t *init_tables,
                          const ModelInit *init, uint32_t *queue, uint32_t *status, int unit, TailTask *tails,
-                         uint32_t *tail_count) {
-  compress_fast_loop<8>(tasks, ntasks, slots, init_tables, init, queue, status, unit, tails, tail_count);
+                         uint32_t *tail_count, uint32_t roles) {
+  compress_fast_loop<8>(tasks, ntasks, slots, init_tables, init, queue, status, unit, tails, tail_count, roles);
 }
 
 // Units of 160..256 bits.
 __global__ void __launch_bounds__(kFastThreads, 2)
     compress_fast_kernel_wide(const ChunkTask *tasks, uint32_t ntasks, uint8_t *slots, const uint8_t *init_tables,
                               const ModelInit *init, uint32_t *queue, uint32_t *status, int unit, TailTask *tails,
-                              uint32_t *tail_count) {
-  compress_fast_loop<16>(tasks, ntasks, slots, init_tables, init, queue, status, unit, tails, tail_count);
+                              uint32_t *tail_count, uint32_t roles) {
+  compress_fast_loop<16>(tasks, ntasks, slots, init_tables, init, queue, status, unit, tails, tail_count, roles);
 }
 
 // One chunk, task passed by value, tables at `slot` (no work queue); the
@@ -783,7 +918,7 @@ __global__ void __launch_bounds__(kFastThreads, 2)
   const FastSmem s = carve_fast(smem_raw, L);
   copy_tables(&g_tables, s.tab);
   __syncthreads();
-  compress_fast_one<GR>(t, slot, s, L, init, status, nullptr, nullptr);
+  compress_fast_one<GR>(t, slot, s, L, init, status, nullptr, nullptr, kRolesAlone);
 }
 
 // The tail pass: one thread per handed-over chunk codes its stale tail (the

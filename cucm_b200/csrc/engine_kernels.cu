@@ -626,15 +626,17 @@ cudaError_t launch_compress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t *
                             TailTask *tails, uint32_t *tail_count) {
   if (unit <= kFastMaxUnit && !cfg.generic) {
     const size_t smem = make_fast_layout(unit).total;
+    const uint32_t sms = (uint32_t)(cfg.sm_count > 0 ? cfg.sm_count : 148);
+    const uint32_t roles = nslots <= sms ? kRolesAlone : kRolesPaired;
     const void *kern = unit <= 128 ? (const void *)compress_fast_kernel : (const void *)compress_fast_kernel_wide;
     cudaError_t e = set_smem(kern, smem);
     if (e != cudaSuccess) return e;
     if (unit <= 128)
       compress_fast_kernel<<<nslots, kFastThreads, smem, stream>>>(d_tasks, ntasks, slots, init_tables, d_init,
-                                                                    d_queue, d_status, unit, tails, tail_count);
+                                                                    d_queue, d_status, unit, tails, tail_count, roles);
     else
       compress_fast_kernel_wide<<<nslots, kFastThreads, smem, stream>>>(d_tasks, ntasks, slots, init_tables, d_init,
-                                                                         d_queue, d_status, unit, tails, tail_count);
+                                                                         d_queue, d_status, unit, tails, tail_count, roles);
     e = cudaGetLastError();
     if (e != cudaSuccess || !tails) return e;
     const int lanes = coder_lanes(ntasks, cfg.sm_count);
