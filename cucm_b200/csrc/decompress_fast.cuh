@@ -9,41 +9,57 @@
 //
 // The decoding warp:
 //   * gives the 15 nodes of the nibble's speculation tree (every prefix of
-//     0..3 bits) their 8 context keys and frozen slot states -- one lane per
-//     node, its 6 hashed orders' gathers in flight together (orders 0 and 1
-//     come from shared memory when the CTA has room for them), so a round
-//     costs one memory round trip;
+//     0..3 bits) their 8 context keys and frozen slot states -- two lanes per
+//     node, the even and the odd orders, the 6 hashed orders' gathers in
+//     flight together (orders 0 and 1 come from shared memory when the CTA has
+//     room for them), so a round costs one memory round trip;
 //   * mixes and squashes each node's prediction against the frozen model
-//     (probabilities kept stretched) and decodes the 4 bits uniformly (every
-//     lane runs the same coder arithmetic; the split point of a node comes
-//     from its lane by shuffle);
-//   * has the 4 lanes on the decoded path record keys, states and mixer
-//     inputs of their bit in a per-unit ring, and publishes the round.
-// The updating warp follows one round behind (lane = order), polling for
-// published rounds: the bit-history walk through a per-unit overlay (slot ->
-// live state, 4-key buckets), the StateMap probability chain and the mixer
-// deltas, all in bit order.  Nothing the decoding warp reads changes before
-// the unit ends, so the two only meet there: the overlay's states go to the
-// slot tables, the live probabilities become the frozen ones and the summed
-// mixer deltas join the weights (updateStateMap / updateMixer,
+//     (probabilities kept stretched) and decodes the 4 bits, a lane per leaf of
+//     the tree (dec_nibble);
+//   * issues the next round's gathers, then has the lanes on the decoded path
+//     record keys, states and mixer inputs of their bit in a per-unit ring,
+//     and publishes the round.
+// The updating warp follows, polling for published rounds, all four bits and
+// eight orders of a round at once (dec_update_round): live states through a
+// hash of the unit's keys, the StateMap probabilities and the mixer deltas.
+// Nothing the decoding warp reads changes before the unit ends, so the two
+// only meet there: the unit's last state of every slot goes to the slot
+// tables, the live probabilities become the frozen ones and the summed mixer
+// deltas join the weights (updateStateMap / updateMixer,
 // cucm_decompress_v2.cu:870-896).  Rounds never straddle a unit or byte
 // boundary: units are multiples of 32 bits.
+//
+// A round of one of 16 chunks takes 2,290 cycles: ~1,450 from the first gather
+// to the last byte back (a single random gather from HBM takes 900, the
+// slowest of 90 about 1,450; with 256 chunks ~1,800), ~360 to decode, ~250 for
+// the next keys and gathers, ~160 to mix; recording and the coder state's
+// broadcast run under the gathers.
 //
 // Several warp pairs of a CTA decode independent chunks and share the
 // read-only tables.
 
 constexpr int kDecMaxUnit = 256;
-constexpr int kDecMaxPairs = 8;          // chunks per CTA
+constexpr int kDecMaxPairs = 8;          // chunks per CTA (5 for units above 64 bits: 740 chunks' tables are 142 GB)
 constexpr int kDecWin = 2048;            // payload window per chunk (bytes)
 constexpr int kDecNodes = 15;            // nodes of a 4-bit speculation tree
 constexpr size_t kDecSmemLimit = 227 * 1024;  // dynamic shared memory of one CTA
 constexpr uint32_t kDecSpinLimit = 1u << 27;  // default bound on the updater's polls for a round (seconds)
 
+// Everything a chunk keeps per order -- probabilities, weights, records -- is
+// in columns: even orders in columns 0..3, odd ones in 4..7, the halves that
+// the decoding warp's half warps take.
+__host__ __device__ constexpr int dec_order(int col) { return 2 * (col & 3) + (col >> 2); }
+
+// Row lengths of the [column][state] arrays: the columns' rows start in
+// different banks.
+constexpr int kDecSplRow = 260, kDecSpfRow = 264;
+constexpr uint32_t kDecNone = 0xffu;  // no position (positions that are looked up end at 251)
+
 struct DecLayout {
-  int U, NS, logNS, warps, rounds;
+  int U, NT, logNT, warps, rounds;
   bool low;  // order 0/1 tables held in shared memory
-  size_t off_spf, off_spl, off_w, off_dw, off_ovk, off_ovs, off_ovl, off_ovn, off_prog, off_rk, off_rs, off_rsmp,
-      off_rpc, off_win, off_outb, off_t01, per_warp, off_tab, total;
+  size_t off_spf, off_spl, off_w, off_dw, off_ovt, off_och, off_ons, off_prog, off_rk, off_rs, off_rsmp, off_rpc,
+      off_win, off_outb, off_t01, per_warp, off_tab, total;
 };
 
 // Shared memory of `warps` chunks (warp pairs) and the shared tables.
@@ -54,8 +70,8 @@ __host__ __device__ inline DecLayout make_dec_layout(int U, int warps, bool low 
   L.U = U;
   L.low = low;
   L.rounds = U / 4;
-  L.NS = next_pow2(2 * U);  // overlay slots per order (load <= 1/2)
-  L.logNS = ilog2(L.NS);
+  L.NT = next_pow2(2 * U);
+  L.logNT = ilog2(L.NT);
   L.warps = warps;
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -63,16 +79,15 @@ __host__ __device__ inline DecLayout make_dec_layout(int U, int warps, bool low 
     o = (o + bytes + 15) & ~(size_t)15;
     return at;
   };
-  L.off_spf = take(sizeof(int16_t) * 256 * kOrders);           // frozen probability, stretched [state][order]
-  L.off_spl = take(sizeof(uint32_t) * 256 * kOrders);          // live statep [state][order]
+  L.off_spf = take(sizeof(int16_t) * kOrders * kDecSpfRow);    // frozen probability, stretched [column][state]
+  L.off_spl = take(sizeof(uint32_t) * kOrders * kDecSplRow);   // live statep [column][state]
   L.off_w = take(sizeof(int32_t) * kMixCtx * kOrders);         // frozen weights
   L.off_dw = take(sizeof(int32_t) * kMixCtx * kOrders);        // summed deltas of the unit
-  L.off_ovk = take(sizeof(uint32_t) * kOrders * L.NS);         // overlay keys + 1 (0 = empty), 4-key buckets
-  L.off_ovs = take((size_t)kOrders * L.NS);                    // overlay live states
-  L.off_ovl = take(sizeof(uint16_t) * U * kOrders);            // overlay entries in use [entry][order]
-  L.off_ovn = take(sizeof(int) * kOrders);
+  L.off_ovt = take((size_t)kOrders * L.NT);                    // last position with a key hash [column][hash]
+  L.off_och = take((size_t)U * kOrders);                       // position before it with that hash [bit][column]
+  L.off_ons = take((size_t)U * kOrders);                       // state the bit left in its slot [bit][column]
   L.off_prog = take(sizeof(uint32_t) * 4);                     // rounds published; task index
-  L.off_rk = take(sizeof(uint32_t) * L.rounds * 4 * kOrders);  // records [round][bit][order]
+  L.off_rk = take(sizeof(uint32_t) * L.rounds * 4 * kOrders);  // records [round][bit][column]
   L.off_rs = take((size_t)L.rounds * 4 * kOrders);
   L.off_rsmp = take(sizeof(int16_t) * L.rounds * 4 * kOrders);
   L.off_rpc = take(sizeof(uint32_t) * L.rounds * 4);           // pr | cxt << 16 | y << 24
@@ -89,10 +104,7 @@ struct DecSmem {
   int16_t *spf;
   uint32_t *spl;
   int32_t *w, *dw;
-  uint32_t *ovk;
-  uint8_t *ovs;
-  uint16_t *ovl;
-  int *ovn;
+  uint8_t *ovt, *och, *ons;
   volatile uint32_t *prog;
   uint32_t *rk;
   uint8_t *rs;
@@ -109,10 +121,9 @@ __device__ inline DecSmem carve_dec(uint8_t *base, const DecLayout &L, int warp)
   s.spl = reinterpret_cast<uint32_t *>(b + L.off_spl);
   s.w = reinterpret_cast<int32_t *>(b + L.off_w);
   s.dw = reinterpret_cast<int32_t *>(b + L.off_dw);
-  s.ovk = reinterpret_cast<uint32_t *>(b + L.off_ovk);
-  s.ovs = b + L.off_ovs;
-  s.ovl = reinterpret_cast<uint16_t *>(b + L.off_ovl);
-  s.ovn = reinterpret_cast<int *>(b + L.off_ovn);
+  s.ovt = b + L.off_ovt;
+  s.och = b + L.off_och;
+  s.ons = b + L.off_ons;
   s.prog = reinterpret_cast<volatile uint32_t *>(b + L.off_prog);
   s.rk = reinterpret_cast<uint32_t *>(b + L.off_rk);
   s.rs = b + L.off_rs;
@@ -136,224 +147,320 @@ __device__ __forceinline__ uint32_t ld_slot_state(const uint8_t *p) {
 // Warp-wide refill of the payload window so that it starts at or just below
 // payload byte `at`, on a 16-byte boundary of the payload's address (so the
 // window base may lie up to 15 bytes before the payload).  Only 16-byte
-// blocks that hold payload bytes are read.  Returns the payload offset of
-// window byte 0.
+// blocks that hold payload bytes are read; bytes past the payload are 255, as
+// the reference's decoder shifts them in.  Returns the payload offset of window
+// byte 0.
 __device__ inline long long dec_refill(uint8_t *win, const uint8_t *pay, uint64_t plen, uint64_t at, int lane) {
   const uint8_t *a = reinterpret_cast<const uint8_t *>((reinterpret_cast<uintptr_t>(pay) + at) & ~(uintptr_t)15);
   const uint8_t *end = pay + plen;
+  __syncwarp();  // (every lane has read what it needs of the old window)
   for (int j = lane; j < kDecWin / 16; j += 32) {
     const uint8_t *blk = a + 16 * j;
-    if (blk < end) *reinterpret_cast<uint4 *>(win + 16 * j) = *reinterpret_cast<const uint4 *>(blk);
+    uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
+    if (blk < end) {
+      v = *reinterpret_cast<const uint4 *>(blk);
+      const int have = end - blk < 16 ? (int)(end - blk) : 16;
+      auto past = [&](int w) -> uint32_t {  // mask of word w's bytes past the payload
+        const int n = have - 4 * w;
+        return n >= 4 ? 0u : n <= 0 ? ~0u : ~0u << (8 * n);
+      };
+      v.x |= past(0);
+      v.y |= past(1);
+      v.z |= past(2);
+      v.w |= past(3);
+    }
+    *reinterpret_cast<uint4 *>(win + 16 * j) = v;
   }
   __syncwarp();
   return (long long)(a - pay);
 }
 
-// Overlay buckets hold 4 keys (+ 1, 0 = empty), filled in order and never
-// emptied within a unit; a key whose bucket is full lives in the next bucket
-// with room.  Place of `want` in bucket q, or -1:
-__device__ __forceinline__ int bucket_place(const uint4 &q, uint32_t want) {
-  return q.x == want ? 0 : q.y == want ? 1 : q.z == want ? 2 : q.w == want ? 3 : -1;
-}
-__device__ __forceinline__ int bucket_used(const uint4 &q) {
-  return (q.x != 0u) + (q.y != 0u) + (q.z != 0u) + (q.w != 0u);
+// The window's next four bytes from offset `at`, first byte highest.
+__device__ __forceinline__ uint32_t dec_next4(const uint8_t *win, uint32_t at) {
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(win) + (at >> 2);
+  return __byte_perm(__funnelshift_r(w[0], w[1], 8 * (at & 3)), 0, 0x0123);
 }
 
-// Model update of one round's 4 bits for order `o` (one lane per order), in
-// bit order: the live state of each slot (overlay, else the frozen state the
-// prediction saw), its next state, the StateMap probability of the live state
-// (cucm_decompress_v2.cu:870-883) and the mixer deltas (:885-896).
+// Coder state of a decoding warp, identical in every lane.
+struct DecCoder {
+  uint32_t x1, x2, x;
+  uint64_t ioff;   // payload bytes taken
+  long long wbase; // payload offset of the window's first byte
+};
+
+// Decodes 4 bits along the speculation tree (cucm_decompress_v2.cu:813-868)
+// and returns them, first bit highest.  f_node: lane n (n < 15) holds node n's
+// probability << 20; next: the payload's next four bytes.
 //
-// All shared-memory reads of the four bits are issued before any write:
-// what an earlier bit of the round changes for a later one -- the same
-// slot's state, the same state's probability, an overlay entry it claims --
-// is carried forward in registers, and the writes follow in bit order, so a
-// later write to the same place wins as it would one bit at a time.
-// `nov` is this lane's count of overlay entries in use (its order's list).
-__device__ __forceinline__ void dec_update_round(const DecSmem &s, const Tables *tab, const DecLayout &L, int o,
-                                                 int rd, int &nov) {
-  uint32_t *ovk = s.ovk + o * L.NS;
-  uint8_t *ovs = s.ovs + o * L.NS;
-  const uint32_t bmask = (uint32_t)(L.NS / 4 - 1);
-  uint32_t k[4], b[4], e[4] = {0, 0, 0, 0};
-  int fz[4], sm[4], y[4];
-  int cx[4], dl[4];
+// Lanes 0..15 (16..31 the same again) each run the coder down one leaf's path,
+// taking its bits for granted and checking them against x on the side; one
+// lane's check holds.  No step waits for a comparison, a shuffle or a branch: a
+// bit shifts by 0 or 8, and where one of the first three has to shift further
+// (seen in `least`) the nibble is decoded bit by bit instead.  The nibble is
+// known before the path's state is: `settle` brings that to all lanes, once
+// the next round's gathers are out.  Bit by bit the nibble took 340 cycles.
+struct DecPath {
+  uint32_t x1, x2, x, taken;  // of this lane's path, before the last bit's shift
+  int leaf;                   // the path decoded, -1: the coder state is final already
+};
+
+__device__ __forceinline__ uint32_t dec_nibble(DecCoder &c, DecPath &w, uint32_t f_node, uint32_t next,
+                                               const uint8_t *win, int lane) {
+  const int p = lane & 15;
+  uint32_t f[4];
+  f[0] = __shfl_sync(0xffffffffu, f_node, 0);
+  f[1] = __shfl_sync(0xffffffffu, f_node, 1 + (p >> 3));
+  f[2] = __shfl_sync(0xffffffffu, f_node, 3 + (p >> 2));
+  f[3] = __shfl_sync(0xffffffffu, f_node, 7 + (p >> 1));
+  uint32_t x1 = c.x1, x2 = c.x2, x = c.x, nb = next, least = 0xffffffffu, taken = 0;
+  bool ok = true;
 CUCM_UNROLL
   for (int i = 0; i < 4; i++) {
-    const int r = (rd * 4 + i) * kOrders + o;
-    k[i] = s.rk[r];
-    fz[i] = s.rs[r];
-    sm[i] = s.rsmp[r];
-    const uint32_t pc = s.rpc[rd * 4 + i];
-    y[i] = (int)(pc >> 24) & 1;
-    const int pr = (int)(pc & 0xffffu);
-    cx[i] = (int)(pc >> 16) & 0xff;
-    dl[i] = (int)(((long long)(((y[i] << 12) - pr) * 7) * sm[i]) >> 16);
-    b[i] = bucket_of(k[i], L.logNS - 2);
+    const uint32_t n = ((p >> (3 - i)) & 1) - 1u;  // all ones for a 0
+    const uint32_t t = __umulhi(x2 - x1, f[i]);
+    const uint32_t xm = x1 + t, xn = x1 + t + 1;
+    ok = ok && ((x <= xm) == (n == 0u));
+    x2 = (x2 & n) | (xm & ~n);
+    x1 = (xn & n) | (x1 & ~n);
+    if (i == 3) break;
+    const uint32_t d = x1 ^ x2;
+    least = min(least, d);
+    const uint32_t s = d < 0x1000000u ? 8u : 0u;
+    x1 <<= s;
+    x2 = __funnelshift_l(0xffffffffu, x2, s);
+    x = __funnelshift_l(nb, x, s);
+    nb <<= s;
+    taken += s;
   }
-  // mixer deltas (Mixer::update, cucm_compress_v2.cu:663-678): this lane
-  // alone owns column o of the delta rows; deltas of the round's bits that
-  // share a row are summed first (integer adds commute), then every distinct
-  // row is read and written once
-  bool merged[4] = {false, false, false, false};
-CUCM_UNROLL
-  for (int i = 1; i < 4; i++)
-CUCM_UNROLL
-    for (int j = 0; j < i; j++)
-      if (!merged[i] && !merged[j] && cx[j] == cx[i]) {
-        dl[j] += dl[i];
-        merged[i] = true;
-      }
-  int dv[4];
-CUCM_UNROLL
-  for (int i = 0; i < 4; i++) dv[i] = s.dw[cx[i] * kOrders + o];
-  // the four bits' buckets: keys and states
-  const uint4 *ovk4 = reinterpret_cast<const uint4 *>(ovk);
-  const uint32_t *ovs4 = reinterpret_cast<const uint32_t *>(ovs);
-  uint4 q[4];
-  uint32_t qs[4];
-CUCM_UNROLL
+  const uint32_t hit = __ballot_sync(0xffffffffu, ok);
+  const uint32_t far = __ballot_sync(0xffffffffu, ok && least < 0x10000u);
+  // the lane with the check, in tests side by side (a find-first is ~20 cycles)
+  const uint32_t leaf = ((hit & 0xff00u) ? 8u : 0u) | ((hit & 0xf0f0u) ? 4u : 0u) | ((hit & 0xccccu) ? 2u : 0u) |
+                        ((hit & 0xaaaau) ? 1u : 0u);
+  w.x1 = x1;
+  w.x2 = x2;
+  w.x = x;
+  w.taken = taken;
+  w.leaf = (int)leaf;
+  if (!far) return leaf;
+  uint32_t nib = 0;
+  int n = 0;
+#pragma unroll 1
   for (int i = 0; i < 4; i++) {
-    q[i] = ovk4[b[i]];
-    qs[i] = ovs4[b[i]];
-  }
-  // slots and live states, in bit order; e = slot (bucket * 4 + place)
-  int live[4], ns[4];
-  bool fresh[4];
-CUCM_UNROLL
-  for (int i = 0; i < 4; i++) {
-    bool same = false;
-    int lv = 0;
-CUCM_UNROLL
-    for (int j = 0; j < i; j++)
-      if (k[j] == k[i]) {
-        same = true;
-        lv = ns[j];
-        e[i] = e[j];
-      }
-    fresh[i] = false;
-    if (!same) {
-      const uint32_t want = k[i] + 1;
-      const int hit = bucket_place(q[i], want);
-      if (hit >= 0) {
-        e[i] = b[i] * 4 + (uint32_t)hit;
-        lv = (int)(qs[i] >> (8 * hit)) & 0xff;
-      } else {
-        // places this round has already claimed in the bucket
-        int used = bucket_used(q[i]);
-CUCM_UNROLL
-        for (int j = 0; j < i; j++) used += (fresh[j] && (e[j] >> 2) == b[i]);
-        if (used < 4) {
-          e[i] = b[i] * 4 + (uint32_t)used;
-          lv = fz[i];
-          fresh[i] = true;
-        } else {
-          // full bucket: the key is in a later one, or goes to the first
-          // with room
-          uint32_t bi = b[i];
-          for (uint32_t it = 0; it <= bmask; it++) {
-            bi = (bi + 1) & bmask;
-            const uint4 qq = ovk4[bi];
-            const int h = bucket_place(qq, want);
-            if (h >= 0) {
-              e[i] = bi * 4 + (uint32_t)h;
-              lv = ovs[e[i]];
-              break;
-            }
-            int u = bucket_used(qq);
-CUCM_UNROLL
-            for (int j = 0; j < i; j++) u += (fresh[j] && (e[j] >> 2) == bi);
-            if (u < 4) {
-              e[i] = bi * 4 + (uint32_t)u;
-              lv = fz[i];
-              fresh[i] = true;
-              break;
-            }
-          }
-        }
-      }
+    const uint32_t xm = c.x1 + __umulhi(c.x2 - c.x1, __shfl_sync(0xffffffffu, f_node, n));
+    const int y = c.x <= xm;
+    if (y) c.x2 = xm; else c.x1 = xm + 1;
+    while ((c.x1 ^ c.x2) < 0x1000000u) {
+      c.x1 <<= 8;
+      c.x2 = (c.x2 << 8) | 255u;
+      c.x = (c.x << 8) | (uint32_t)win[(long long)c.ioff - c.wbase];
+      c.ioff++;
     }
-    live[i] = lv;
-    ns[i] = tab->nex[lv][y[i]];
+    nib = (nib << 1) | (uint32_t)y;
+    n = 2 * n + 1 + y;
   }
-  // StateMap probabilities of the live states: a state met m times earlier
-  // in the round has count min(count + m, 1023), so every dt is read up front
-  uint32_t v0[4], dtv[4];
-  int m[4];
-CUCM_UNROLL
-  for (int i = 0; i < 4; i++) {
-    v0[i] = s.spl[live[i] * kOrders + o];
-    m[i] = 0;
-CUCM_UNROLL
-    for (int j = 0; j < i; j++) m[i] += (live[j] == live[i]);
-    const uint32_t c = (v0[i] & 1023u) + (uint32_t)m[i];
-    dtv[i] = tab->dt[c > 1023u ? 1023u : c];
-  }
-  uint32_t nv[4];
-CUCM_UNROLL
-  for (int i = 0; i < 4; i++) {
-    uint32_t v = v0[i];
-CUCM_UNROLL
-    for (int j = 0; j < i; j++)
-      if (live[j] == live[i]) v = nv[j];
-    nv[i] = statep_next(v, y[i], dtv[i]);
-  }
-  // writes, in bit order
-CUCM_UNROLL
-  for (int i = 0; i < 4; i++)
-    if (!merged[i]) s.dw[cx[i] * kOrders + o] = dv[i] + dl[i];
-CUCM_UNROLL
-  for (int i = 0; i < 4; i++) {
-    if (fresh[i]) {
-      ovk[e[i]] = k[i] + 1;
-      s.ovl[nov * kOrders + o] = (uint16_t)e[i];
-      nov++;
-    }
-    ovs[e[i]] = (uint8_t)ns[i];
-    s.spl[live[i] * kOrders + o] = nv[i];
+  w.leaf = -1;
+  return nib;
+}
+
+__device__ __forceinline__ void dec_settle(DecCoder &c, const DecPath &w, const uint8_t *win) {
+  if (w.leaf < 0) return;
+  c.x1 = __shfl_sync(0xffffffffu, w.x1, w.leaf);
+  c.x2 = __shfl_sync(0xffffffffu, w.x2, w.leaf);
+  c.x = __shfl_sync(0xffffffffu, w.x, w.leaf);
+  c.ioff += __shfl_sync(0xffffffffu, w.taken, w.leaf) >> 3;
+  while ((c.x1 ^ c.x2) < 0x1000000u) {  // the last bit's shift
+    c.x1 <<= 8;
+    c.x2 = (c.x2 << 8) | 255u;
+    c.x = (c.x << 8) | (uint32_t)win[(long long)c.ioff - c.wbase];
+    c.ioff++;
   }
 }
 
-// Unit end, both warps of the pair (t = 0..63): overlay -> slot tables (and
-// cleared), live probabilities become frozen (stretched for the mixer),
-// deltas join the weights, the unit's bytes go out.  Called between two pair
-// barriers.
-__device__ inline void dec_unit_end(const DecSmem &s, const DecLayout &L, const Tables *tab, uint8_t *slot,
-                                    uint8_t *out, int nbytes, int t) {
+// `if (mine) *at = v`, in program order with the other such stores of the
+// warp: where lanes share an address, the last one's value stays.
+__device__ __forceinline__ void store_turn8(bool mine, uint32_t at, uint32_t v) {
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.u8 [%1], %2; }" ::"r"((uint32_t)mine), "r"(at), "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ void store_turn32(bool mine, uint32_t at, uint32_t v) {
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.u32 [%1], %2; }" ::"r"((uint32_t)mine), "r"(at),
+               "r"(v)
+               : "memory");
+}
+
+// Model update of one round's 4 bits (lane = column lane & 7, bit lane >> 3):
+// the live state of each slot (what an earlier bit of the unit left there, else
+// the frozen state the prediction saw), its next state, the StateMap
+// probability of the live state in bit order (cucm_decompress_v2.cu:870-883)
+// and the mixer deltas (:885-896).
+//
+// A bit's key is looked up among the unit's earlier ones through a small hash
+// of the last position per key hash, positions with the same hash chained
+// backwards through och.  Nothing is cleared between units: a position at or
+// past this round's is left from the unit before and ends a search, one before
+// it holds a key of this unit, which is compared.  The four keys of a round
+// and an order differ (they share the previous bytes; the hash is one-to-one
+// in the partial byte), so the lookups do not depend on one another; only bits
+// that meet the same state of the same order wait for each other.  A slot's
+// earlier record is marked (bit 31 of its key): the unit end writes the
+// unmarked ones.
+//
+// All shared-memory reads stand before the writes (the compiler keeps their
+// order).  One lane per order, its four bits after one another, took 2,000
+// cycles a round, more than the decoding warp's 120 gathers.
+__device__ __forceinline__ void dec_update_round(const DecSmem &s, const Tables *tab, const DecLayout &L, int lane,
+                                                 int rd) {
+  const int o = lane & 7, i = lane >> 3;
+  const uint32_t base = 4u * (uint32_t)rd, j = base + (uint32_t)i;
+  const int r = 32 * rd + lane;
+  const uint32_t k = s.rk[r];
+  const uint32_t fz = s.rs[r];
+  const int sm = s.rsmp[r];
+  const uint32_t pc = s.rpc[4 * rd + i];
+  const int y = (int)(pc >> 24) & 1, pr = (int)(pc & 0xffffu);
+  const uint32_t cx = (pc >> 16) & 0xffu;
+  const int delta = (int)(((long long)(((y << 12) - pr) * 7) * sm) >> 16);
+  const uint32_t h = bucket_of(k, L.logNT);
+  uint8_t *last = s.ovt + o * L.NT + h;
+  const uint32_t p = *last;
+  // the search: most end at the first position
+  bool more = p < base;
+  uint32_t q = more ? p : 0u, found = kDecNone;
+  {
+    const uint32_t kk = s.rk[q * kOrders + o], c = s.och[q * kOrders + o];
+    if (more && kk == k) found = q;
+    more = more && kk != k && c < q;
+    q = more ? c : 0u;
+  }
+  while (__any_sync(0xffffffffu, more)) {
+    const uint32_t kk = s.rk[q * kOrders + o], c = s.och[q * kOrders + o];
+    if (more && kk == k) found = q;
+    more = more && kk != k && c < q;
+    q = more ? c : 0u;
+  }
+  const bool again = found != kDecNone;
+  const uint32_t left = s.ons[(again ? found : 0u) * kOrders + o];
+  const uint32_t live = again ? left : fz;
+  const uint32_t next = tab->nex[live][y];
+  uint32_t v = s.spl[o * kDecSplRow + live];
+  // positions of this round with the same hash
+  const uint32_t h1 = __shfl_up_sync(0xffffffffu, h, 8), h2 = __shfl_up_sync(0xffffffffu, h, 16),
+                 h3 = __shfl_up_sync(0xffffffffu, h, 24);
+  uint32_t before = p < base ? p : kDecNone;
+  if (i >= 3 && h3 == h) before = j - 3;
+  if (i >= 2 && h2 == h) before = j - 2;
+  if (i >= 1 && h1 == h) before = j - 1;
+  // a state met m times earlier in the round has count min(count + m, 1023)
+  const uint32_t l0 = __shfl_sync(0xffffffffu, live, o), l1 = __shfl_sync(0xffffffffu, live, o + 8),
+                 l2 = __shfl_sync(0xffffffffu, live, o + 16);
+  const bool e0 = i > 0 && l0 == live, e1 = i > 1 && l1 == live, e2 = i > 2 && l2 == live;
+  const uint32_t m = (uint32_t)e0 + (uint32_t)e1 + (uint32_t)e2;
+  const uint32_t rate = tab->dt[min((v & 1023u) + m, 1023u)];
+  uint32_t nv = statep_next(v, y, rate);
+  if (__any_sync(0xffffffffu, m != 0)) {
+    const uint32_t n0 = __shfl_sync(0xffffffffu, nv, o);
+    v = e0 ? n0 : v;
+    nv = statep_next(v, y, rate);
+    const uint32_t n1 = __shfl_sync(0xffffffffu, nv, o + 8);
+    v = e1 ? n1 : v;
+    nv = statep_next(v, y, rate);
+    const uint32_t n2 = __shfl_sync(0xffffffffu, nv, o + 16);
+    v = e2 ? n2 : v;
+    nv = statep_next(v, y, rate);
+  }
+  // writes; where bits share a place, the later bit's stays
+  if (again) s.rk[found * kOrders + o] = k | 0x80000000u;
+  s.ons[r] = (uint8_t)next;
+  s.och[r] = (uint8_t)before;
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(last);
+  const uint32_t sp = (uint32_t)__cvta_generic_to_shared(s.spl + o * kDecSplRow + live);
 CUCM_UNROLL
-  for (int o = 0; o < kOrders; o++) {
-    const int n = s.ovn[o];
+  for (int t = 0; t < 4; t++) {
+    store_turn8(i == t, at, j);
+    store_turn32(i == t, sp, nv);
+  }
+  atomicAdd(&s.dw[cx * kOrders + o], delta);
+  __syncwarp();
+}
+
+// Unit end, both warps of the pair (t = 0..63): the slots' last states go to
+// the slot tables, live probabilities become frozen (stretched for the mixer),
+// deltas join the weights, the unit's bytes go out.  Called between two pair
+// barriers.  Reads are issued in batches ahead of the writes.
+__device__ inline void dec_unit_end(const DecSmem &s, const DecLayout &L, const Tables *tab, uint8_t *slot,
+                                    uint8_t *out, int nbits, int t) {
+  {
+    const int o = dec_order(t & 7);
     uint8_t *tb = (o < 2 && s.t01 ? s.t01 : slot) + table_offset(o);
-    for (int e = t; e < n; e += 64) {
-      const int b = s.ovl[e * kOrders + o];
-      const uint32_t kk = s.ovk[o * L.NS + b];
-      tb[kk - 1] = s.ovs[o * L.NS + b];
-      s.ovk[o * L.NS + b] = 0;
+    for (int e0 = t; e0 < nbits * kOrders; e0 += 64 * 8) {
+      uint32_t kk[8], ns[8];
+CUCM_UNROLL
+      for (int i = 0; i < 8; i++) {
+        const int e = e0 + 64 * i;
+        const bool in = e < nbits * kOrders;
+        kk[i] = in ? s.rk[e] : 0x80000000u;
+        ns[i] = in ? s.ons[e] : 0u;
+      }
+CUCM_UNROLL
+      for (int i = 0; i < 8; i++)
+        if (!(kk[i] >> 31)) tb[kk[i]] = (uint8_t)ns[i];
     }
   }
-  const uint4 *src = reinterpret_cast<const uint4 *>(s.spl);
-  uint2 *dst = reinterpret_cast<uint2 *>(s.spf);
   const int16_t *str = tab->stretch;
-#pragma unroll 4
-  for (int i = t; i < 256 * kOrders / 4; i += 64) {
-    const uint4 q = src[i];
-    const uint32_t a = (uint16_t)str[q.x >> 20], b = (uint16_t)str[q.y >> 20];
-    const uint32_t c = (uint16_t)str[q.z >> 20], d = (uint16_t)str[q.w >> 20];
-    dst[i] = make_uint2(a | (b << 16), c | (d << 16));
+CUCM_UNROLL
+  for (int h = 0; h < 2; h++) {
+    uint4 q[4];
+    uint2 d[4];
+CUCM_UNROLL
+    for (int i = 0; i < 4; i++) {  // column 4h + i, states 4t .. 4t + 3
+      q[i] = *reinterpret_cast<const uint4 *>(s.spl + (4 * h + i) * kDecSplRow + 4 * t);
+    }
+CUCM_UNROLL
+    for (int i = 0; i < 4; i++) {
+      const uint32_t a = (uint16_t)str[q[i].x >> 20], b = (uint16_t)str[q[i].y >> 20];
+      const uint32_t c = (uint16_t)str[q[i].z >> 20], e = (uint16_t)str[q[i].w >> 20];
+      d[i] = make_uint2(a | (b << 16), c | (e << 16));
+    }
+CUCM_UNROLL
+    for (int i = 0; i < 4; i++) *reinterpret_cast<uint2 *>(s.spf + (4 * h + i) * kDecSpfRow + 4 * t) = d[i];
   }
   int4 *w4 = reinterpret_cast<int4 *>(s.w);
   int4 *d4 = reinterpret_cast<int4 *>(s.dw);
-  for (int i = t; i < kMixCtx * kOrders / 4; i += 64) {
-    int4 a = w4[i];
-    const int4 d = d4[i];
-    a.x += d.x;
-    a.y += d.y;
-    a.z += d.z;
-    a.w += d.w;
-    w4[i] = a;
-    d4[i] = make_int4(0, 0, 0, 0);
+  int4 a[3], d[3];
+CUCM_UNROLL
+  for (int i = 0; i < 3; i++) {
+    const int e = t + 64 * i;
+    if (e < kMixCtx * kOrders / 4) {
+      a[i] = w4[e];
+      d[i] = d4[e];
+    }
   }
-  if (t < nbytes) out[t] = s.outb[t];
+CUCM_UNROLL
+  for (int i = 0; i < 3; i++) {
+    const int e = t + 64 * i;
+    if (e < kMixCtx * kOrders / 4) {
+      w4[e] = make_int4(a[i].x + d[i].x, a[i].y + d[i].y, a[i].z + d[i].z, a[i].w + d[i].w);
+      d4[e] = make_int4(0, 0, 0, 0);
+    }
+  }
+  if (t < (nbits >> 3)) out[t] = s.outb[t];
+}
+
+// Mixer output of one node (Mixer::p, cucm_compress_v2.cu:636-644, then pr++
+// below 2048, which the decoder's copy of the squash table already holds), the
+// half warps with four orders each.  |sum| < 2^45, so sum >> 16 fits 32 bits.
+__device__ __forceinline__ uint32_t dec_mix(const int32_t *w, int cxt, const int smp[4], int half,
+                                            const uint16_t *squash) {
+  const int4 a = reinterpret_cast<const int4 *>(w)[2 * cxt + half];
+  const long long s0 = (long long)a.x * smp[0] + (long long)a.y * smp[1];
+  const long long s1 = (long long)a.z * smp[2] + (long long)a.w * smp[3];
+  long long sum = s0 + s1;
+  const uint32_t lo = __shfl_xor_sync(0xffffffffu, (uint32_t)sum, 16);
+  const uint32_t hi = __shfl_xor_sync(0xffffffffu, (uint32_t)(sum >> 32), 16);
+  sum += (long long)((uint64_t)lo | ((uint64_t)hi << 32));
+  const int idx = (int)(sum >> 16);
+  return squash[max(-2047, min(2048, idx)) + 2047];
 }
 
 // The pair's barrier: named barrier 1 + pair index, 64 threads.
@@ -375,22 +482,22 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
   const uint64_t plen = t.in_len;
 
   for (int i = t64; i < 256 * kOrders; i += 64) {
-    const uint32_t v = init->statep[i & 7][i >> 3];
-    s.spf[i] = tab->stretch[v >> 20];
-    s.spl[i] = v;
+    const int col = i >> 8, st = i & 255;
+    const uint32_t v = init->statep[dec_order(col)][st];
+    s.spf[col * kDecSpfRow + st] = tab->stretch[v >> 20];
+    s.spl[col * kDecSplRow + st] = v;
   }
   for (int i = t64; i < kMixCtx * kOrders; i += 64) {
-    s.w[i] = init->w[i];
+    s.w[i] = init->w[(i & ~7) + dec_order(i & 7)];
     s.dw[i] = 0;
   }
-  for (int i = t64; i < kOrders * L.NS; i += 64) s.ovk[i] = 0;
+  for (int i = t64; i < kOrders * L.NT; i += 64) s.ovt[i] = (uint8_t)kDecNone;
   if (kLow) {
     // the chunk's order 0/1 tables move to shared memory for its lifetime
     const uint4 *src = reinterpret_cast<const uint4 *>(slot);
     uint4 *dst = reinterpret_cast<uint4 *>(s.t01);
     for (int i = t64; i < (int)(kHashedOff / 16); i += 64) dst[i] = src[i];
   }
-  if (t64 < kOrders) s.ovn[t64] = 0;
   if (t64 == 0) s.prog[0] = 0;
   pair_sync(pair);
 
@@ -400,7 +507,6 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
     bool ok = true;
     for (uint64_t base = 0; base < nbits; base += (uint64_t)U) {
       const int nunit = (int)(nbits - base < (uint64_t)U ? nbits - base : (uint64_t)U);
-      int nov = 0;
       for (int rd = 0; rd < (nunit >> 2); rd++) {
         uint32_t spins = 0;
         while (ok && s.prog[0] <= done) {
@@ -410,33 +516,41 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
         }
         __threadfence_block();
         if (!ok) break;
-        if (lane < kOrders) dec_update_round(s, tab, L, lane, rd, nov);
+        dec_update_round(s, tab, L, lane, rd);
         done++;
       }
-      if (lane < kOrders) s.ovn[lane] = nov;
       if (!ok && lane == 0) atomicOr(status, (uint32_t)kDevTimeout);
       pair_sync(pair);
-      dec_unit_end(s, L, tab, slot, t.out + (base >> 3), nunit >> 3, t64);
+      dec_unit_end(s, L, tab, slot, t.out + (base >> 3), nunit, t64);
       pair_sync(pair);
     }
     return;
   }
 
-  long long wbase = dec_refill(s.win, pay, plen, 0, lane);
+  DecCoder c;
+  c.wbase = dec_refill(s.win, pay, plen, 0, lane);
 
-  // coder state, identical in every lane (cucm_decompress_v2.cu:967-972)
-  uint32_t x1 = 0, x2 = 0xffffffffu, x = 0;
-  uint64_t ioff = 0;
-  for (int i = 0; i < 4; i++, ioff++) x = (x << 8) | (ioff < plen ? (uint32_t)s.win[(long long)ioff - wbase] : 255u);
+  // coder state (cucm_decompress_v2.cu:967-972)
+  c.x1 = 0;
+  c.x2 = 0xffffffffu;
+  c.x = dec_next4(s.win, (uint32_t)(0 - c.wbase));
+  c.ioff = 4;
 
-  // node of this lane (lanes 15..31 mirror lanes 0..14 so every gather
-  // instruction stays uniform; only lanes < 15 record)
-  const int node = lane % kDecNodes;
+  // node of this lane: each half warp holds the 15 nodes (its last lane doubles
+  // the last one), the lower half their even orders, the upper half the odd
+  // ones, so that a round takes three gather instructions of 30 lines
+  const int half = lane >> 4;
+  const int node = (lane & 15) < kDecNodes ? lane & 15 : kDecNodes - 1;
   const int depth = 31 - __clz(node + 1);
   const uint32_t pbits = (uint32_t)(node + 1 - (1 << depth));
-  const bool recorder = lane < kDecNodes;
+  const bool recorder = (lane & 15) < kDecNodes;
+  const int16_t *spf = s.spf + 4 * half * kDecSpfRow;
+  const uint8_t *low = kLow ? s.t01 + (half ? kOrder1Off : 0) : slot + (half ? kOrder1Off : 0);
+  const uint8_t *tables[3];
+CUCM_UNROLL
+  for (int q = 0; q < 3; q++) tables[q] = slot + table_offset(2 * q + 2 + half);
 
-  uint64_t hist = 0;  // completed bytes, most recent in the low byte
+  uint32_t hist[7] = {0, 0, 0, 0, 0, 0, 0};  // completed bytes, most recent first
   uint32_t cur = 0;   // bits of the current byte
   int r = 0;          // 0 or 4
   uint32_t published = 0;
@@ -445,98 +559,76 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
   // next round's gathers go out at once (within a unit: the unit end writes
   // the slot tables), and the decoded round is recorded and published while
   // they are in flight.
-  BitKeys kk;
-  uint32_t st[kOrders];
-  auto gather = [&](BitKeys &k, uint32_t *sv, uint32_t cur_, int r_, uint64_t hist_) {
-    const uint32_t h0 = (1u << (r_ + depth)) | (cur_ << depth) | pbits;
-    bit_keys64(h0, hist_, k);
-    if (kLow) {
-      sv[0] = s.t01[k.k[0]];
-      sv[1] = s.t01[kOrder1Off + k.k[1]];
-    }
+  uint32_t kk[4], st[4];
+  uint32_t next = 0;  // the payload's next four bytes
+  auto gather = [&]() {
+    const uint32_t h0 = (1u << (r + depth)) | (cur << depth) | pbits;
+    BitKeys k;
+    bit_keys(h0, hist, k);
 CUCM_UNROLL
-    for (int o = kLow ? 2 : 0; o < kOrders; o++) sv[o] = ld_slot_state(slot + table_offset(o) + k.k[o]);
+    for (int q = 0; q < 4; q++) kk[q] = half ? k.k[2 * q + 1] : k.k[2 * q];
+    if (kLow) st[0] = low[kk[0]];
+CUCM_UNROLL
+    for (int q = 0; q < 3; q++) st[q + 1] = ld_slot_state(tables[q] + kk[q + 1]);
+    if (!kLow) st[0] = ld_slot_state(low + kk[0]);
+  };
+  // while the gathers are in flight: the payload window
+  auto ahead = [&]() {
+    if ((long long)c.ioff + 16 > c.wbase + kDecWin) c.wbase = dec_refill(s.win, pay, plen, c.ioff, lane);
+    next = dec_next4(s.win, (uint32_t)((long long)c.ioff - c.wbase));
   };
 
   for (uint64_t base = 0; base < nbits; base += (uint64_t)U) {
     const int nunit = (int)(nbits - base < (uint64_t)U ? nbits - base : (uint64_t)U);
     const int nr = nunit >> 2;
     int obyte = 0;
-    gather(kk, st, cur, r, hist);
+    gather();
+    ahead();
     for (int rd = 0; rd < nr; rd++) {
-      if ((long long)ioff + 16 > wbase + kDecWin) wbase = dec_refill(s.win, pay, plen, ioff, lane);
       // stretch, mixer context, mixer output (cucm_decompress_v2.cu:774-809)
-      const int c1 = (int)(hist & 0xffu);
-      int smp[kOrders];
+      int smp[4];
       int olen = 0;
 CUCM_UNROLL
-      for (int o = 0; o < kOrders; o++) {
-        smp[o] = s.spf[st[o] * kOrders + o];
-        olen += (smp[o] != 1);
-      }
-      const int cxt = olen + (c1 >> 5) * 10;
-      const int pr_node = mix_pr(s.w, cxt, smp, tab);
-      // decode 4 bits along the tree (cucm_decompress_v2.cu:813-868); both
-      // children's split factors are fetched while a bit is decided, so the
-      // shuffle is off the bit-to-bit chain
-      const uint32_t f_node = (uint32_t)pr_node << 20;
-      int n = 0;
-      uint32_t nib = 0;
-      uint32_t f = __shfl_sync(0xffffffffu, f_node, 0);
+      for (int q = 0; q < 4; q++) smp[q] = spf[q * kDecSpfRow + st[q]];
 CUCM_UNROLL
-      for (int i = 0; i < 4; i++) {
-        uint32_t fa = 0, fb = 0;
-        if (i < 3) {
-          fa = __shfl_sync(0xffffffffu, f_node, 2 * n + 1);
-          fb = __shfl_sync(0xffffffffu, f_node, 2 * n + 2);
-        }
-        const uint32_t xm = x1 + __umulhi(x2 - x1, f);
-        const int y = x <= xm;
-        if (y) x2 = xm; else x1 = xm + 1;
-        while ((x1 ^ x2) < 0x1000000u) {
-          x1 <<= 8;
-          x2 = (x2 << 8) | 255u;
-          x = (x << 8) | (ioff < plen ? (uint32_t)s.win[(long long)ioff - wbase] : 255u);
-          ioff++;
-        }
-        nib = (nib << 1) | (uint32_t)y;
-        n = 2 * n + 1 + y;
-        f = y ? fb : fa;
-      }
+      for (int q = 0; q < 4; q++) olen += (smp[q] != 1);
+      olen += __shfl_xor_sync(0xffffffffu, olen, 16);
+      const int cxt = olen + (int)(hist[0] >> 5) * 10;
+      const uint32_t pr_node = dec_mix(s.w, cxt, smp, half, tab->squash);
+      DecPath path;
+      const uint32_t nib = dec_nibble(c, path, pr_node << 20, next, s.win, lane);
       // the round's record, kept in registers while the next round's
       // gathers go out
       const bool on_path = recorder && pbits == (nib >> (4 - depth));
-      const uint4 rk0 = make_uint4(kk.k[0], kk.k[1], kk.k[2], kk.k[3]);
-      const uint4 rk1 = make_uint4(kk.k[4], kk.k[5], kk.k[6], kk.k[7]);
-      const uint2 rsv = make_uint2(st[0] | (st[1] << 8) | (st[2] << 16) | (st[3] << 24),
-                                   st[4] | (st[5] << 8) | (st[6] << 16) | (st[7] << 24));
-      const uint4 rm = make_uint4((uint32_t)(smp[0] & 0xffff) | ((uint32_t)smp[1] << 16),
-                                  (uint32_t)(smp[2] & 0xffff) | ((uint32_t)smp[3] << 16),
-                                  (uint32_t)(smp[4] & 0xffff) | ((uint32_t)smp[5] << 16),
-                                  (uint32_t)(smp[6] & 0xffff) | ((uint32_t)smp[7] << 16));
-      const uint32_t rpc = (uint32_t)pr_node | ((uint32_t)cxt << 16) | (((nib >> (3 - depth)) & 1u) << 24);
+      const uint4 rk = make_uint4(kk[0], kk[1], kk[2], kk[3]);
+      const uint32_t rsv = st[0] | (st[1] << 8) | (st[2] << 16) | (st[3] << 24);
+      const uint2 rm = make_uint2((uint32_t)(smp[0] & 0xffff) | ((uint32_t)smp[1] << 16),
+                                  (uint32_t)(smp[2] & 0xffff) | ((uint32_t)smp[3] << 16));
+      const uint32_t rpc = pr_node | ((uint32_t)cxt << 16) | (((nib >> (3 - depth)) & 1u) << 24);
       cur = (cur << 4) | nib;
       r += 4;
       bool byte_done = false;
       if (r == 8) {
         byte_done = true;
-        hist = (hist << 8) | cur;
+CUCM_UNROLL
+        for (int i = 6; i > 0; i--) hist[i] = hist[i - 1];
+        hist[0] = cur;
         cur = 0;
         r = 0;
       }
-      if (rd + 1 < nr) gather(kk, st, cur, r, hist);
+      if (rd + 1 < nr) gather();
+      dec_settle(c, path, s.win);
+      ahead();
       // the path's lanes record their bit for the updating warp
       if (on_path) {
-        const int i = depth;
-        uint4 *k4 = reinterpret_cast<uint4 *>(s.rk + (rd * 4 + i) * kOrders);
-        k4[0] = rk0;
-        k4[1] = rk1;
-        *reinterpret_cast<uint2 *>(s.rs + (rd * 4 + i) * kOrders) = rsv;
-        *reinterpret_cast<uint4 *>(s.rsmp + (rd * 4 + i) * kOrders) = rm;
-        s.rpc[rd * 4 + i] = rpc;
+        const int e = (rd * 4 + depth) * kOrders + 4 * half;
+        *reinterpret_cast<uint4 *>(s.rk + e) = rk;
+        *reinterpret_cast<uint32_t *>(s.rs + e) = rsv;
+        *reinterpret_cast<uint2 *>(s.rsmp + e) = rm;
+        if (half == 0) s.rpc[rd * 4 + depth] = rpc;
       }
       if (byte_done) {
-        if (lane == 0) s.outb[obyte] = (uint8_t)hist;
+        if (lane == 0) s.outb[obyte] = (uint8_t)hist[0];
         obyte++;
       }
       __syncwarp();
@@ -547,7 +639,7 @@ CUCM_UNROLL
       }
     }
     pair_sync(pair);
-    dec_unit_end(s, L, tab, slot, t.out + (base >> 3), nunit >> 3, t64);
+    dec_unit_end(s, L, tab, slot, t.out + (base >> 3), nunit, t64);
     pair_sync(pair);
   }
 }
@@ -564,6 +656,8 @@ __global__ void __launch_bounds__(kDecMaxPairs * 64)
   const DecLayout L = make_dec_layout(unit, pairs, kLow);
   Tables *tab = reinterpret_cast<Tables *>(smem_raw + L.off_tab);
   copy_tables(&g_tables, tab);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4096; i += blockDim.x) tab->squash[i] += tab->squash[i] < 2048;  // see dec_mix
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = warp >> 1, role = warp & 1;

@@ -659,7 +659,8 @@ static int dec_max_pairs(int unit) {
   const DecLayout one = make_dec_layout(unit, 1);
   const size_t avail = kDecSmemLimit - (one.total - one.per_warp);
   int w = (int)(avail / one.per_warp);
-  return w < 1 ? 1 : (w > kDecMaxPairs ? kDecMaxPairs : w);
+  const int cap = unit > 64 ? 5 : kDecMaxPairs;
+  return w < 1 ? 1 : (w > cap ? cap : w);
 }
 
 static bool dec_fast(int unit, const EngineConfig &cfg) { return unit <= kDecMaxUnit && !cfg.generic; }
