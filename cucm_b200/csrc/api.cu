@@ -808,6 +808,8 @@ int cucm_compress_dev(cucm_ctx *c, const uint8_t *in, uint64_t n, const cucm_par
   return compress_containers(c, 1, &in, &n, p, &out, &cap, out_n, &st, true);
 }
 
+constexpr uint64_t kFramingHead = 4096;
+
 // Decompress `count` containers (decompress, cucm_decompress_v2.cu:1185-1248,
 // per container).  Containers without a prelearn prefix are decoded in one
 // engine run per unit length; a prelearn prefix means its own model and run.
@@ -815,7 +817,10 @@ static int decompress_containers(cucm_ctx *c, uint32_t count, const uint8_t *con
                                  uint8_t *const *outs, const uint64_t *caps, uint64_t *out_ns, int *status, bool dev) {
   std::lock_guard<std::mutex> g(c->mu);
   CK(cudaSetDevice(c->device));
-  // The header, prelearn block and batch framing are parsed on the host.
+  // The header, prelearn block and batch framing are parsed on the host.  Of a
+  // container in device memory only those are fetched: its first bytes, which
+  // mostly hold all of them, then what lies further on.  (The whole of it, by
+  // way of pageable memory, took 26 ms of a 811 ms call over 64 MiB.)
   std::vector<std::vector<uint8_t>> host_copy(dev ? count : 0);
   std::vector<const uint8_t *> h(count);
   std::vector<Parsed> ph(count);
@@ -827,8 +832,8 @@ static int decompress_containers(cucm_ctx *c, uint32_t count, const uint8_t *con
     if (status[i]) continue;
     h[i] = ins[i];
     if (dev) {
-      host_copy[i].resize(ns[i]);
-      CK(cudaMemcpy(host_copy[i].data(), ins[i], ns[i], cudaMemcpyDeviceToHost));
+      host_copy[i].resize(std::min<uint64_t>(ns[i], kFramingHead));
+      CK(cudaMemcpy(host_copy[i].data(), ins[i], host_copy[i].size(), cudaMemcpyDeviceToHost));
       h[i] = host_copy[i].data();
     }
     status[i] = parse_header(h[i], ns[i], ph[i]);
@@ -841,8 +846,21 @@ static int decompress_containers(cucm_ctx *c, uint32_t count, const uint8_t *con
     const uint64_t body_off = ph[i].body_off();
     const uint64_t out_body = ph[i].total - ph[i].prelearn;
     const uint64_t nchunks = (out_body + ph[i].cs - 1) / ph[i].cs;
-    status[i] = parse_batches(h[i] + body_off, ns[i] - body_off, nchunks, ph[i].batch, true, off[i], len[i],
-                              ph[i].wide);
+    if (dev && ph[i].prelearn && body_off > host_copy[i].size()) {
+      const uint64_t have = host_copy[i].size();
+      host_copy[i].resize(body_off);
+      CK(cudaMemcpy(host_copy[i].data() + have, ins[i] + have, body_off - have, cudaMemcpyDeviceToHost));
+      h[i] = host_copy[i].data();
+    }
+    std::vector<uint8_t> piece;
+    auto read = [&](uint64_t at, uint64_t bytes) -> const uint8_t * {
+      at += body_off;
+      if (!dev || at + bytes <= host_copy[i].size()) return h[i] + at;
+      piece.resize(bytes);
+      return cudaMemcpy(piece.data(), ins[i] + at, bytes, cudaMemcpyDeviceToHost) == cudaSuccess ? piece.data() : nullptr;
+    };
+    status[i] = parse_batches_from(read, ns[i] - body_off, nchunks, ph[i].batch, true, off[i], len[i], ph[i].wide);
+    if (status[i] == CUCM_ECUDA) return CUCM_ECUDA;
     if (!status[i]) ok.push_back(i);
   }
   // groups: one per unit length for model-free containers, one per prelearned container

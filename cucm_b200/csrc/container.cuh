@@ -236,8 +236,12 @@ inline int parse_header(const uint8_t *in, uint64_t n, Parsed &h) {
 
 // Chunk payload extents of the batches that follow the prelearn block
 // (cucm_decompress_v2.cu:1223-1237).  Offsets are relative to `body`.
-inline int parse_batches(const uint8_t *body, uint64_t body_n, uint64_t nchunks, uint32_t batch, bool with_sizes,
-                         std::vector<uint64_t> &off, std::vector<uint64_t> &len, bool wide = false) {
+// read(off, n) gives n bytes of the body from `off` (inside it), or null when
+// they cannot be fetched; a batch's size field and its table are read, its
+// payloads are not.
+template <class Read>
+inline int parse_batches_from(Read read, uint64_t body_n, uint64_t nchunks, uint32_t batch, bool with_sizes,
+                              std::vector<uint64_t> &off, std::vector<uint64_t> &len, bool wide) {
   off.resize(nchunks);
   len.resize(nchunks);
   const uint64_t w = wide ? 8 : 4;
@@ -248,7 +252,9 @@ inline int parse_batches(const uint8_t *body, uint64_t body_n, uint64_t nchunks,
     uint64_t bsz;
     if (with_sizes) {
       if (r + w > body_n) return CUCM_EFORMAT;
-      bsz = get_le(body + r, wide);
+      const uint8_t *size = read(r, w);
+      if (!size) return CUCM_ECUDA;
+      bsz = get_le(size, wide);
       r += w;
     } else {
       bsz = body_n - r;
@@ -257,8 +263,10 @@ inline int parse_batches(const uint8_t *body, uint64_t body_n, uint64_t nchunks,
     const uint64_t pay0 = r + w * C;
     const uint64_t pay_n = bsz - w * C;
     uint64_t start = 0;
+    const uint8_t *table = read(r, w * C);
+    if (!table) return CUCM_ECUDA;
     for (uint64_t k = k0; k < k1; k++) {
-      uint64_t endv = get_be(body + r + w * (k - k0), wide);
+      uint64_t endv = get_be(table + w * (k - k0), wide);
       if (endv + 1 < w * C) return CUCM_EFORMAT;
       uint64_t end = endv + 1 - w * C;
       if (end < start || end > pay_n) return CUCM_EFORMAT;
@@ -269,6 +277,11 @@ inline int parse_batches(const uint8_t *body, uint64_t body_n, uint64_t nchunks,
     r += bsz;
   }
   return CUCM_OK;
+}
+inline int parse_batches(const uint8_t *body, uint64_t body_n, uint64_t nchunks, uint32_t batch, bool with_sizes,
+                         std::vector<uint64_t> &off, std::vector<uint64_t> &len, bool wide = false) {
+  return parse_batches_from([&](uint64_t at, uint64_t) { return body + at; }, body_n, nchunks, batch, with_sizes, off,
+                            len, wide);
 }
 
 // Batch layout of n chunks (cudaencodefinal,
