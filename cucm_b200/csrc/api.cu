@@ -262,6 +262,7 @@ int run_engine(cucm_ctx *c, bool decode, std::vector<ChunkTask> &tasks, int unit
     CK(cudaEventRecord(fork, c->stream));
     for (uint32_t s = 0; s < S; s++) CK(cudaStreamWaitEvent(c->side[s], fork, 0));
     const uint8_t *img = ms.image ? c->image.as<uint8_t>() : nullptr;
+    cfg.others = S - 1;
     for (uint32_t i = 0; i < n; i++) {
       uint32_t s = i % S;
       uint8_t *slot = c->slots.as<uint8_t>() + (size_t)s * kSlotTableBytes;

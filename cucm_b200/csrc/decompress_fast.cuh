@@ -384,61 +384,68 @@ CUCM_UNROLL
   __syncwarp();
 }
 
-// Unit end, both warps of the pair (t = 0..63): the slots' last states go to
-// the slot tables, live probabilities become frozen (stretched for the mixer),
-// deltas join the weights, the unit's bytes go out.  Called between two pair
+// Unit end, kThreads threads (t = 0..kThreads - 1): the slots' last states go
+// to the slot tables, live probabilities become frozen (stretched for the
+// mixer), deltas join the weights, the unit's bytes go out.  Called between two
 // barriers.  Reads are issued in batches ahead of the writes.
+template <int kThreads>
 __device__ inline void dec_unit_end(const DecSmem &s, const DecLayout &L, const Tables *tab, uint8_t *slot,
                                     uint8_t *out, int nbits, int t) {
+  constexpr int kSlots8 = kThreads >= 256 ? 2 : 8;  // slots of a thread's batch
   {
     const int o = dec_order(t & 7);
     uint8_t *tb = (o < 2 && s.t01 ? s.t01 : slot) + table_offset(o);
-    for (int e0 = t; e0 < nbits * kOrders; e0 += 64 * 8) {
-      uint32_t kk[8], ns[8];
+    for (int e0 = t; e0 < nbits * kOrders; e0 += kThreads * kSlots8) {
+      uint32_t kk[kSlots8], ns[kSlots8];
 CUCM_UNROLL
-      for (int i = 0; i < 8; i++) {
-        const int e = e0 + 64 * i;
+      for (int i = 0; i < kSlots8; i++) {
+        const int e = e0 + kThreads * i;
         const bool in = e < nbits * kOrders;
         kk[i] = in ? s.rk[e] : 0x80000000u;
         ns[i] = in ? s.ons[e] : 0u;
       }
 CUCM_UNROLL
-      for (int i = 0; i < 8; i++)
+      for (int i = 0; i < kSlots8; i++)
         if (!(kk[i] >> 31)) tb[kk[i]] = (uint8_t)ns[i];
     }
   }
   const int16_t *str = tab->stretch;
+  constexpr int kQuads = kThreads >= 256 ? 1 : 4;  // groups of four states of a thread's batch
+  for (int i0 = t; i0 < 64 * kOrders; i0 += kThreads * kQuads) {
+    uint4 q[kQuads];
+    uint2 d[kQuads];
 CUCM_UNROLL
-  for (int h = 0; h < 2; h++) {
-    uint4 q[4];
-    uint2 d[4];
-CUCM_UNROLL
-    for (int i = 0; i < 4; i++) {  // column 4h + i, states 4t .. 4t + 3
-      q[i] = *reinterpret_cast<const uint4 *>(s.spl + (4 * h + i) * kDecSplRow + 4 * t);
+    for (int i = 0; i < kQuads; i++) {
+      const int g = min(i0 + kThreads * i, 64 * kOrders - 1);
+      q[i] = *reinterpret_cast<const uint4 *>(s.spl + (g >> 6) * kDecSplRow + 4 * (g & 63));
     }
 CUCM_UNROLL
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < kQuads; i++) {
       const uint32_t a = (uint16_t)str[q[i].x >> 20], b = (uint16_t)str[q[i].y >> 20];
       const uint32_t c = (uint16_t)str[q[i].z >> 20], e = (uint16_t)str[q[i].w >> 20];
       d[i] = make_uint2(a | (b << 16), c | (e << 16));
     }
 CUCM_UNROLL
-    for (int i = 0; i < 4; i++) *reinterpret_cast<uint2 *>(s.spf + (4 * h + i) * kDecSpfRow + 4 * t) = d[i];
+    for (int i = 0; i < kQuads; i++) {
+      const int g = i0 + kThreads * i;
+      if (g < 64 * kOrders) *reinterpret_cast<uint2 *>(s.spf + (g >> 6) * kDecSpfRow + 4 * (g & 63)) = d[i];
+    }
   }
   int4 *w4 = reinterpret_cast<int4 *>(s.w);
   int4 *d4 = reinterpret_cast<int4 *>(s.dw);
-  int4 a[3], d[3];
+  constexpr int kRows = (kMixCtx * kOrders / 4 + kThreads - 1) / kThreads;
+  int4 a[kRows], d[kRows];
 CUCM_UNROLL
-  for (int i = 0; i < 3; i++) {
-    const int e = t + 64 * i;
+  for (int i = 0; i < kRows; i++) {
+    const int e = t + kThreads * i;
     if (e < kMixCtx * kOrders / 4) {
       a[i] = w4[e];
       d[i] = d4[e];
     }
   }
 CUCM_UNROLL
-  for (int i = 0; i < 3; i++) {
-    const int e = t + 64 * i;
+  for (int i = 0; i < kRows; i++) {
+    const int e = t + kThreads * i;
     if (e < kMixCtx * kOrders / 4) {
       w4[e] = make_int4(a[i].x + d[i].x, a[i].y + d[i].y, a[i].z + d[i].z, a[i].w + d[i].w);
       d4[e] = make_int4(0, 0, 0, 0);
@@ -463,6 +470,141 @@ __device__ __forceinline__ uint32_t dec_mix(const int32_t *w, int cxt, const int
   return squash[max(-2047, min(2048, idx)) + 2047];
 }
 
+// A lane of a warp that predicts the nodes of a speculation tree.  Each half
+// warp holds the 15 nodes (its last lane doubles the last one), the lower half
+// their even orders, the upper half the odd ones, so that a round takes three
+// gather instructions of 30 lines.
+template <bool kLow>
+struct DecLane {
+  int half, depth;
+  uint32_t pbits;
+  bool recorder;
+  const int16_t *spf;
+  const uint8_t *low;
+  const uint8_t *tables[3];
+
+  __device__ __forceinline__ DecLane(const DecSmem &s, const uint8_t *slot, int lane) {
+    half = lane >> 4;
+    const int node = (lane & 15) < kDecNodes ? lane & 15 : kDecNodes - 1;
+    depth = 31 - __clz(node + 1);
+    pbits = (uint32_t)(node + 1 - (1 << depth));
+    recorder = (lane & 15) < kDecNodes;
+    spf = s.spf + 4 * half * kDecSpfRow;
+    low = (kLow ? s.t01 : slot) + (half ? kOrder1Off : 0);
+CUCM_UNROLL
+    for (int q = 0; q < 3; q++) tables[q] = slot + table_offset(2 * q + 2 + half);
+  }
+
+  // Keys and frozen slot states of this lane's node and orders, r bits `cur`
+  // into the byte after `hist`.
+  __device__ __forceinline__ void gather(uint32_t cur, int r, const uint32_t hist[7], uint32_t kk[4],
+                                         uint32_t st[4]) const {
+    const uint32_t h0 = (1u << (r + depth)) | (cur << depth) | pbits;
+    BitKeys k;
+    bit_keys(h0, hist, k);
+CUCM_UNROLL
+    for (int q = 0; q < 4; q++) kk[q] = half ? k.k[2 * q + 1] : k.k[2 * q];
+    if (kLow) st[0] = low[kk[0]];
+CUCM_UNROLL
+    for (int q = 0; q < 3; q++) st[q + 1] = ld_slot_state(tables[q] + kk[q + 1]);
+    if (!kLow) st[0] = ld_slot_state(low + kk[0]);
+  }
+
+  // Stretch, mixer context, mixer output (cucm_decompress_v2.cu:774-809).
+  __device__ __forceinline__ uint32_t predict(const DecSmem &s, const Tables *tab, const uint32_t st[4], uint32_t c1,
+                                              int smp[4], int &cxt) const {
+    int olen = 0;
+CUCM_UNROLL
+    for (int q = 0; q < 4; q++) smp[q] = spf[q * kDecSpfRow + st[q]];
+CUCM_UNROLL
+    for (int q = 0; q < 4; q++) olen += (smp[q] != 1);
+    olen += __shfl_xor_sync(0xffffffffu, olen, 16);
+    cxt = olen + (int)(c1 >> 5) * 10;
+    return dec_mix(s.w, cxt, smp, half, tab->squash);
+  }
+};
+
+// What a lane records of its node for the updating warp, if the node is on the
+// path of the nibble decoded.
+struct DecRecord {
+  bool mine;
+  uint4 key;
+  uint32_t state;
+  uint2 smp;
+  uint32_t pc;  // pr | cxt << 16 | y << 24
+};
+
+template <bool kLow>
+__device__ __forceinline__ DecRecord dec_record(const DecLane<kLow> &ln, const uint32_t kk[4], const uint32_t st[4],
+                                                const int smp[4], uint32_t pr, int cxt, uint32_t nib) {
+  DecRecord r;
+  r.mine = ln.recorder && ln.pbits == (nib >> (4 - ln.depth));
+  r.key = make_uint4(kk[0], kk[1], kk[2], kk[3]);
+  r.state = st[0] | (st[1] << 8) | (st[2] << 16) | (st[3] << 24);
+  r.smp = make_uint2((uint32_t)(smp[0] & 0xffff) | ((uint32_t)smp[1] << 16),
+                     (uint32_t)(smp[2] & 0xffff) | ((uint32_t)smp[3] << 16));
+  r.pc = pr | ((uint32_t)cxt << 16) | (((nib >> (3 - ln.depth)) & 1u) << 24);
+  return r;
+}
+
+template <bool kLow>
+__device__ __forceinline__ void dec_write_record(const DecSmem &s, const DecLane<kLow> &ln, const DecRecord &r,
+                                                 int rd) {
+  if (r.mine) {
+    const int e = (rd * 4 + ln.depth) * kOrders + 4 * ln.half;
+    *reinterpret_cast<uint4 *>(s.rk + e) = r.key;
+    *reinterpret_cast<uint32_t *>(s.rs + e) = r.state;
+    *reinterpret_cast<uint2 *>(s.rsmp + e) = r.smp;
+    if (ln.half == 0) s.rpc[rd * 4 + ln.depth] = r.pc;
+  }
+}
+
+// A chunk's model at its start, by kThreads threads.
+template <bool kLow, int kThreads>
+__device__ __forceinline__ void dec_start(const DecSmem &s, const DecLayout &L, const Tables *tab,
+                                          const ModelInit *init, const uint8_t *slot, int t) {
+  for (int i = t; i < 256 * kOrders; i += kThreads) {
+    const int col = i >> 8, st = i & 255;
+    const uint32_t v = init->statep[dec_order(col)][st];
+    s.spf[col * kDecSpfRow + st] = tab->stretch[v >> 20];
+    s.spl[col * kDecSplRow + st] = v;
+  }
+  for (int i = t; i < kMixCtx * kOrders; i += kThreads) {
+    s.w[i] = init->w[(i & ~7) + dec_order(i & 7)];
+    s.dw[i] = 0;
+  }
+  for (int i = t; i < kOrders * L.NT; i += kThreads) s.ovt[i] = (uint8_t)kDecNone;
+  if (kLow) {
+    // the chunk's order 0/1 tables move to shared memory for its lifetime
+    const uint4 *src = reinterpret_cast<const uint4 *>(slot);
+    uint4 *dst = reinterpret_cast<uint4 *>(s.t01);
+    for (int i = t; i < (int)(kHashedOff / 16); i += kThreads) dst[i] = src[i];
+  }
+}
+
+// Coder state of a chunk's first bytes (cucm_decompress_v2.cu:967-972).
+__device__ __forceinline__ void dec_open(DecCoder &c, uint8_t *win, const uint8_t *pay, uint64_t plen, int lane) {
+  c.wbase = dec_refill(win, pay, plen, 0, lane);
+  c.x1 = 0;
+  c.x2 = 0xffffffffu;
+  c.x = dec_next4(win, (uint32_t)(0 - c.wbase));
+  c.ioff = 4;
+}
+
+// The payload's next four bytes; the window moves on where it holds less than
+// 16 bytes (a nibble's most, bit by bit).
+__device__ __forceinline__ uint32_t dec_ahead(DecCoder &c, uint8_t *win, const uint8_t *pay, uint64_t plen, int lane) {
+  if ((long long)c.ioff + 16 > c.wbase + kDecWin) c.wbase = dec_refill(win, pay, plen, c.ioff, lane);
+  return dec_next4(win, (uint32_t)((long long)c.ioff - c.wbase));
+}
+
+// The byte after `hist` joins it.
+__device__ __forceinline__ void dec_push(uint32_t hist[7], uint32_t byte) {
+CUCM_UNROLL
+  for (int i = 6; i > 0; i--) hist[i] = hist[i - 1];
+  hist[0] = byte;
+}
+
 // The pair's barrier: named barrier 1 + pair index, 64 threads.
 __device__ __forceinline__ void pair_sync(int pair) {
   asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
@@ -481,23 +623,7 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
   const uint8_t *pay = t.in;
   const uint64_t plen = t.in_len;
 
-  for (int i = t64; i < 256 * kOrders; i += 64) {
-    const int col = i >> 8, st = i & 255;
-    const uint32_t v = init->statep[dec_order(col)][st];
-    s.spf[col * kDecSpfRow + st] = tab->stretch[v >> 20];
-    s.spl[col * kDecSplRow + st] = v;
-  }
-  for (int i = t64; i < kMixCtx * kOrders; i += 64) {
-    s.w[i] = init->w[(i & ~7) + dec_order(i & 7)];
-    s.dw[i] = 0;
-  }
-  for (int i = t64; i < kOrders * L.NT; i += 64) s.ovt[i] = (uint8_t)kDecNone;
-  if (kLow) {
-    // the chunk's order 0/1 tables move to shared memory for its lifetime
-    const uint4 *src = reinterpret_cast<const uint4 *>(slot);
-    uint4 *dst = reinterpret_cast<uint4 *>(s.t01);
-    for (int i = t64; i < (int)(kHashedOff / 16); i += 64) dst[i] = src[i];
-  }
+  dec_start<kLow, 64>(s, L, tab, init, slot, t64);
   if (t64 == 0) s.prog[0] = 0;
   pair_sync(pair);
 
@@ -521,112 +647,49 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
       }
       if (!ok && lane == 0) atomicOr(status, (uint32_t)kDevTimeout);
       pair_sync(pair);
-      dec_unit_end(s, L, tab, slot, t.out + (base >> 3), nunit, t64);
+      dec_unit_end<64>(s, L, tab, slot, t.out + (base >> 3), nunit, t64);
       pair_sync(pair);
     }
     return;
   }
 
   DecCoder c;
-  c.wbase = dec_refill(s.win, pay, plen, 0, lane);
-
-  // coder state (cucm_decompress_v2.cu:967-972)
-  c.x1 = 0;
-  c.x2 = 0xffffffffu;
-  c.x = dec_next4(s.win, (uint32_t)(0 - c.wbase));
-  c.ioff = 4;
-
-  // node of this lane: each half warp holds the 15 nodes (its last lane doubles
-  // the last one), the lower half their even orders, the upper half the odd
-  // ones, so that a round takes three gather instructions of 30 lines
-  const int half = lane >> 4;
-  const int node = (lane & 15) < kDecNodes ? lane & 15 : kDecNodes - 1;
-  const int depth = 31 - __clz(node + 1);
-  const uint32_t pbits = (uint32_t)(node + 1 - (1 << depth));
-  const bool recorder = (lane & 15) < kDecNodes;
-  const int16_t *spf = s.spf + 4 * half * kDecSpfRow;
-  const uint8_t *low = kLow ? s.t01 + (half ? kOrder1Off : 0) : slot + (half ? kOrder1Off : 0);
-  const uint8_t *tables[3];
-CUCM_UNROLL
-  for (int q = 0; q < 3; q++) tables[q] = slot + table_offset(2 * q + 2 + half);
-
+  dec_open(c, s.win, pay, plen, lane);
+  const DecLane<kLow> ln(s, slot, lane);
   uint32_t hist[7] = {0, 0, 0, 0, 0, 0, 0};  // completed bytes, most recent first
   uint32_t cur = 0;   // bits of the current byte
   int r = 0;          // 0 or 4
   uint32_t published = 0;
 
-  // A round's keys and frozen slot states.  After a round is decoded the
-  // next round's gathers go out at once (within a unit: the unit end writes
-  // the slot tables), and the decoded round is recorded and published while
-  // they are in flight.
+  // After a round is decoded the next round's gathers go out at once (within a
+  // unit: the unit end writes the slot tables); the coder state, the payload
+  // window and the decoded round's record follow while they are in flight.
   uint32_t kk[4], st[4];
-  uint32_t next = 0;  // the payload's next four bytes
-  auto gather = [&]() {
-    const uint32_t h0 = (1u << (r + depth)) | (cur << depth) | pbits;
-    BitKeys k;
-    bit_keys(h0, hist, k);
-CUCM_UNROLL
-    for (int q = 0; q < 4; q++) kk[q] = half ? k.k[2 * q + 1] : k.k[2 * q];
-    if (kLow) st[0] = low[kk[0]];
-CUCM_UNROLL
-    for (int q = 0; q < 3; q++) st[q + 1] = ld_slot_state(tables[q] + kk[q + 1]);
-    if (!kLow) st[0] = ld_slot_state(low + kk[0]);
-  };
-  // while the gathers are in flight: the payload window
-  auto ahead = [&]() {
-    if ((long long)c.ioff + 16 > c.wbase + kDecWin) c.wbase = dec_refill(s.win, pay, plen, c.ioff, lane);
-    next = dec_next4(s.win, (uint32_t)((long long)c.ioff - c.wbase));
-  };
-
   for (uint64_t base = 0; base < nbits; base += (uint64_t)U) {
     const int nunit = (int)(nbits - base < (uint64_t)U ? nbits - base : (uint64_t)U);
     const int nr = nunit >> 2;
     int obyte = 0;
-    gather();
-    ahead();
+    ln.gather(cur, r, hist, kk, st);
+    uint32_t next = dec_ahead(c, s.win, pay, plen, lane);
     for (int rd = 0; rd < nr; rd++) {
-      // stretch, mixer context, mixer output (cucm_decompress_v2.cu:774-809)
-      int smp[4];
-      int olen = 0;
-CUCM_UNROLL
-      for (int q = 0; q < 4; q++) smp[q] = spf[q * kDecSpfRow + st[q]];
-CUCM_UNROLL
-      for (int q = 0; q < 4; q++) olen += (smp[q] != 1);
-      olen += __shfl_xor_sync(0xffffffffu, olen, 16);
-      const int cxt = olen + (int)(hist[0] >> 5) * 10;
-      const uint32_t pr_node = dec_mix(s.w, cxt, smp, half, tab->squash);
+      int smp[4], cxt;
+      const uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
       DecPath path;
-      const uint32_t nib = dec_nibble(c, path, pr_node << 20, next, s.win, lane);
-      // the round's record, kept in registers while the next round's
-      // gathers go out
-      const bool on_path = recorder && pbits == (nib >> (4 - depth));
-      const uint4 rk = make_uint4(kk[0], kk[1], kk[2], kk[3]);
-      const uint32_t rsv = st[0] | (st[1] << 8) | (st[2] << 16) | (st[3] << 24);
-      const uint2 rm = make_uint2((uint32_t)(smp[0] & 0xffff) | ((uint32_t)smp[1] << 16),
-                                  (uint32_t)(smp[2] & 0xffff) | ((uint32_t)smp[3] << 16));
-      const uint32_t rpc = pr_node | ((uint32_t)cxt << 16) | (((nib >> (3 - depth)) & 1u) << 24);
+      const uint32_t nib = dec_nibble(c, path, pr << 20, next, s.win, lane);
+      const DecRecord rec = dec_record(ln, kk, st, smp, pr, cxt, nib);
       cur = (cur << 4) | nib;
       r += 4;
       bool byte_done = false;
       if (r == 8) {
         byte_done = true;
-CUCM_UNROLL
-        for (int i = 6; i > 0; i--) hist[i] = hist[i - 1];
-        hist[0] = cur;
+        dec_push(hist, cur);
         cur = 0;
         r = 0;
       }
-      if (rd + 1 < nr) gather();
+      if (rd + 1 < nr) ln.gather(cur, r, hist, kk, st);
       dec_settle(c, path, s.win);
-      ahead();
-      // the path's lanes record their bit for the updating warp
-      if (on_path) {
-        const int e = (rd * 4 + depth) * kOrders + 4 * half;
-        *reinterpret_cast<uint4 *>(s.rk + e) = rk;
-        *reinterpret_cast<uint32_t *>(s.rs + e) = rsv;
-        *reinterpret_cast<uint2 *>(s.rsmp + e) = rm;
-        if (half == 0) s.rpc[rd * 4 + depth] = rpc;
-      }
+      next = dec_ahead(c, s.win, pay, plen, lane);
+      dec_write_record(s, ln, rec, rd);
       if (byte_done) {
         if (lane == 0) s.outb[obyte] = (uint8_t)hist[0];
         obyte++;
@@ -639,7 +702,7 @@ CUCM_UNROLL
       }
     }
     pair_sync(pair);
-    dec_unit_end(s, L, tab, slot, t.out + (base >> 3), nunit, t64);
+    dec_unit_end<64>(s, L, tab, slot, t.out + (base >> 3), nunit, t64);
     pair_sync(pair);
   }
 }

@@ -546,6 +546,7 @@ __global__ void __launch_bounds__(256) decompress_kernel(const ChunkTask *tasks,
 
 #include "compress_fast.cuh"
 #include "decompress_fast.cuh"
+#include "decompress_wide.cuh"
 #include "fixed_model.cuh"
 
 }  // namespace
@@ -688,6 +689,16 @@ cudaError_t launch_decompress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       if (sms <= 0) sms = 1;
     }
+    const uint32_t spin = cfg.spin_limit ? cfg.spin_limit : kDecSpinLimit;
+    // few chunks: an SM each (unless the caller chose a pair decoder's form)
+    if (nslots + cfg.others <= kWideMaxChunks && nslots <= (uint32_t)sms && cfg.dec_pairs == 0 && cfg.dec_tables == 0) {
+      const DecLayout L = make_dec_layout(unit, 1, true);
+      cudaError_t e = set_smem((const void *)decompress_wide_kernel, L.total);
+      if (e != cudaSuccess) return e;
+      decompress_wide_kernel<<<nslots, kWideThreads, L.total, stream>>>(d_tasks, ntasks, slots, init_tables, d_init,
+                                                                        d_queue, d_status, unit, spin);
+      return cudaGetLastError();
+    }
     int wpc = (int)((nslots + (uint32_t)sms - 1) / (uint32_t)sms);
     const int wmax = dec_max_pairs(unit);
     if (cfg.dec_pairs > 0) wpc = cfg.dec_pairs;
@@ -702,7 +713,6 @@ cudaError_t launch_decompress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t
     cudaError_t e = set_smem(kern, L.total);
     if (e != cudaSuccess) return e;
     const uint32_t grid = (nslots + (uint32_t)wpc - 1) / (uint32_t)wpc;
-    const uint32_t spin = cfg.spin_limit ? cfg.spin_limit : kDecSpinLimit;
     if (low)
       decompress_pair_kernel<true><<<grid, wpc * 64, L.total, stream>>>(d_tasks, ntasks, slots, nslots, init_tables,
                                                                         d_init, d_queue, d_status, unit, spin);

@@ -285,6 +285,11 @@ int run_tasks(cucm_server *s, Launch *l, const std::vector<ChunkTask> &tasks) {
   cfg.dec_tables = s->tuning.dec_tables;
   cfg.cmp_ctas = s->tuning.cmp_ctas;
   cfg.spin_limit = s->tuning.dec_spin_limit;
+  // Launches to come share the device: a chunk that has an SM to itself (the
+  // decoder for a few chunks) would leave no room beside it for a compressor
+  // CTA.  32 requests at 2 GB/s offered: p50 0.76-0.98 s without, 0.78-1.27 s
+  // with it.
+  cfg.others = ~0u >> 1;
   std::vector<ChunkTask> order = tasks;
   const bool dec = l->op == CUCM_OP_DECOMPRESS;
   std::stable_sort(order.begin(), order.end(), [&](const ChunkTask &a, const ChunkTask &b) {

@@ -49,3 +49,45 @@ def test_pairs_per_cta(gpu_ctx, oracle_mod, pairs):
         blob = oracle_mod.compress(data, 5000, unit, 0, 100)
         assert gpu_ctx.decompress(blob) == data
     gpu_ctx.set_tuning()
+
+
+@pytest.mark.parametrize("kind", ["text", "random", "walk", "runs"])
+def test_few_chunks(gpu_ctx, oracle_mod, kind):
+    """An SM per chunk: more chunks than slots (tables restored between
+    them), partial units, one byte, and the same through the pair decoder."""
+    data = W.make(kind, 50001, 17).tobytes()
+    for unit in (32, 128, 160, 256):
+        blob = oracle_mod.compress(data, 5003, unit, 0, 100)
+        for tuning in (dict(max_slots=3), dict(max_slots=1), dict(form=cc.FORM_PLAIN), dict(dec_pairs=1)):
+            gpu_ctx.set_tuning(**tuning)
+            assert gpu_ctx.decompress(blob) == data
+    gpu_ctx.set_tuning()
+    for n in (1, 2, 15, 16, 17, 33):
+        assert gpu_ctx.decompress(oracle_mod.compress(data[:n], 5003, 128, 0, 100)) == data[:n]
+
+
+@pytest.mark.parametrize("chunks", [63, 64, 65, 149])
+def test_around_the_switch(gpu_ctx, oracle_mod, chunks):
+    gpu_ctx.set_tuning()
+    data = W.text(chunks * 700 - 3, chunks).tobytes()
+    assert gpu_ctx.decompress(oracle_mod.compress(data, 700, 128, 0, 100)) == data
+
+
+def test_prelearned_few_chunks(gpu_ctx, oracle_mod):
+    gpu_ctx.set_tuning(max_slots=2)
+    data = W.text(60000, 4).tobytes()
+    assert gpu_ctx.decompress(oracle_mod.compress(data, 8000, 128, 9000, 100)) == data
+    gpu_ctx.set_tuning()
+
+
+@pytest.mark.parametrize("pairs", [0, 1, 2])
+def test_waits_that_run_out(gpu_ctx, oracle_mod, pairs):
+    data = W.text(100_000, 21).tobytes()
+    blob = oracle_mod.compress(data, 20000, 128, 0, 100)
+    gpu_ctx.set_tuning(dec_pairs=pairs, dec_spin_limit=1)
+    with pytest.raises(cc.CucmError) as e:
+        gpu_ctx.decompress(blob)
+    assert e.value.status == -7
+    gpu_ctx.set_tuning(dec_pairs=pairs)
+    assert gpu_ctx.decompress(blob) == data
+    gpu_ctx.set_tuning()
