@@ -60,6 +60,21 @@ __device__ __forceinline__ void wide_byte_wait() {
   asm volatile("bar.sync 1, %0;" ::"n"(32 * (1 + kWideGuess)) : "memory");
 }
 
+// Whether first nibble `guess` after byte c1 is likely enough, by the order-1
+// model alone (lane & 3 = bit).
+__device__ __forceinline__ bool wide_follow(const DecSmem &s, const Tables *tab, uint32_t guess, uint32_t c1,
+                                            int lane) {
+  const int i = lane & 3;
+  const uint32_t h0 = (1u << i) | (guess >> (4 - i));
+  const uint32_t state = s.t01[kOrder1Off + ((c1 << 8) | h0)];
+  const int x = s.spf[4 * kDecSpfRow + state];  // column 4 is order 1
+  const int p1 = tab->squash[x + 2047];
+  float p = (float)(((guess >> (3 - i)) & 1u) ? p1 : 4096 - p1) * (1.0f / 4096.0f);
+  p *= __shfl_xor_sync(0xffffffffu, p, 1);
+  p *= __shfl_xor_sync(0xffffffffu, p, 2);
+  return p > kWideLeast;
+}
+
 __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const DecSmem &s, WideSmem &ws,
                                     const Tables *tab, const DecLayout &L, const ModelInit *init, uint32_t *status,
                                     uint32_t spin_limit) {
@@ -143,17 +158,7 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
     } else if (!updates) {
       for (int b = 0; b < nb; b++) {
         const uint32_t nth = bytes + (uint32_t)b, seq = 2 * nth;
-        // this first nibble's probability by the order-1 model alone (lane & 3
-        // = bit): unlikely ones are not followed
-        const int i = lane & 3;
-        const uint32_t h0 = (1u << i) | (guess >> (4 - i));
-        const uint32_t state = s.t01[kOrder1Off + ((hist[0] << 8) | h0)];
-        const int x = s.spf[4 * kDecSpfRow + state];  // column 4 is order 1
-        const int p1 = tab->squash[x + 2047];
-        float p = (float)(((guess >> (3 - i)) & 1u) ? p1 : 4096 - p1) * (1.0f / 4096.0f);
-        p *= __shfl_xor_sync(0xffffffffu, p, 1);
-        p *= __shfl_xor_sync(0xffffffffu, p, 2);
-        const bool follow = p > kWideLeast;
+        const bool follow = wide_follow(s, tab, guess, hist[0], lane);
         int smp[4], cxt = 0;
         uint32_t pr = 0;
         if (follow) {

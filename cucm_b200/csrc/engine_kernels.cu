@@ -560,6 +560,10 @@ size_t decompress_smem_bytes(int unit, int spec_bits) {
   return make_layout(unit, 0).total + kNodeBytes;
 }
 
+static cudaError_t set_smem(const void *fn, size_t bytes) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // Chunks that share a warp of a one-thread-per-chunk coder kernel: one while
 // every chunk can have a warp scheduler of its own (a group that is done again
 // for one lane holds up the warp's others), else just enough.
@@ -590,13 +594,26 @@ cudaError_t launch_fixed_encode(const FixedTask *d_tasks, const uint64_t *d_firs
 cudaError_t launch_fixed_decode(const FixedTask *d_tasks, uint32_t ntasks, const uint8_t *image,
                                 const ModelInit *d_init, uint32_t *d_queue, int sm_count, cudaStream_t stream) {
   if (ntasks == 0) return cudaSuccess;
+  const uint32_t sms = (uint32_t)(sm_count > 0 ? sm_count : 148);
+  // A CTA per chunk while every chunk can have an SM: text in chunks of 16 KiB,
+  // 37.0 -> 24.8 ms with 16 chunks, 36.8 -> 26.5 with 148 (random bytes 37.6 ->
+  // 35.9); two waves of CTAs would not pay.
+  if (ntasks <= sms) {
+    const size_t smem = fixed_dec_smem_bytes(1);
+    cudaError_t e = set_smem((const void *)fixed_decode_wide_kernel, smem);
+    if (e != cudaSuccess) return e;
+    fixed_decode_wide_kernel<<<ntasks, kFixedWideThreads, smem, stream>>>(d_tasks, ntasks, image, d_init, d_queue);
+    return cudaGetLastError();
+  }
   // chunks spread over all SMs first: warps per CTA = chunks per SM, at
   // most kFixedDecWarps (each warp's rounds wait on its gathers, so warps
   // sharing an SM slow each other only through its load pipe)
-  const uint32_t sms = (uint32_t)(sm_count > 0 ? sm_count : 148);
   const uint32_t warps = std::min<uint32_t>(kFixedDecWarps, (ntasks + sms - 1) / sms);
   const uint32_t want = (ntasks + warps - 1) / warps;
-  fixed_decode_kernel<<<std::min(want, sms * 4), warps * 32, 0, stream>>>(d_tasks, ntasks, image, d_init, d_queue);
+  const size_t smem = fixed_dec_smem_bytes((int)warps);
+  cudaError_t e = set_smem((const void *)fixed_decode_kernel, smem);
+  if (e != cudaSuccess) return e;
+  fixed_decode_kernel<<<std::min(want, sms * 2), warps * 32, smem, stream>>>(d_tasks, ntasks, image, d_init, d_queue);
   return cudaGetLastError();
 }
 
@@ -604,10 +621,6 @@ cudaError_t upload_tables() {
   Tables t;
   build_tables(t);
   return cudaMemcpyToSymbol(g_tables, &t, sizeof(Tables));
-}
-
-static cudaError_t set_smem(const void *fn, size_t bytes) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // Pipelined compressor CTAs that fit on one SM: shared memory (1 KiB of it

@@ -23,9 +23,8 @@
 //   fixed_coder_kernel  one thread per chunk runs the arithmetic coder over
 //                       its chunk's array;
 //
-// and the decoder is one warp per chunk decoding a nibble per round over the
-// 15-node speculation tree, the next round's gathers issued as soon as a
-// round is decided.
+// and the decoder gives each chunk a warp, a nibble per round, or in calls with
+// no more chunks than SMs a CTA, a byte per round.
 
 constexpr int kFixedThreads = 256;
 
@@ -160,91 +159,163 @@ CUCM_UNROLL
   if (base > t.out_cap) atomicOr(status, (uint32_t)kDevOverflow);
 }
 
+// The decoders.  The model is only read, so its order 0 and 1 tables, stretched
+// probabilities and weights sit in shared memory once per CTA, in the layout of
+// the adaptive decoder, whose lanes (DecLane) and coder (dec_nibble) these use.
 constexpr int kFixedDecWarps = 8;
+constexpr size_t kFixedDecSpf = kHashedOff, kFixedDecW = kFixedDecSpf + sizeof(int16_t) * kOrders * kDecSpfRow,
+                 kFixedDecTab = kFixedDecW + sizeof(int32_t) * kMixCtx * kOrders,
+                 kFixedDecWin = kFixedDecTab + sizeof(Tables);
+inline size_t fixed_dec_smem_bytes(int windows) { return kFixedDecWin + (size_t)windows * kDecWin; }
 
-// Warp = chunk (tasks handed out by a queue).  Lanes 0..14 are the nodes of
-// the nibble's speculation tree (lanes 15..31 mirror them so every load stays
-// uniform); each gathers its 8 states, mixes, and the warp decodes the 4
-// bits uniformly (cucm_decompress_v2.cu:813-868's coder).  The window of the
-// payload is staged per warp in shared memory.
+__device__ __forceinline__ Tables *fixed_dec_load(uint8_t *smem, const uint8_t *image, const ModelInit *init,
+                                                  DecSmem &s) {
+  s.t01 = smem;
+  s.spf = reinterpret_cast<int16_t *>(smem + kFixedDecSpf);
+  s.w = reinterpret_cast<int32_t *>(smem + kFixedDecW);
+  Tables *tab = reinterpret_cast<Tables *>(smem + kFixedDecTab);
+  copy_tables(&g_tables, tab);
+  const uint4 *src = reinterpret_cast<const uint4 *>(image);
+  for (int i = threadIdx.x; i < (int)(kHashedOff / 16); i += blockDim.x) reinterpret_cast<uint4 *>(s.t01)[i] = src[i];
+  for (int i = threadIdx.x; i < 256 * kOrders; i += blockDim.x)
+    s.spf[(i >> 8) * kDecSpfRow + (i & 255)] = g_tables.stretch[init->statep[dec_order(i >> 8)][i & 255] >> 20];
+  for (int i = threadIdx.x; i < kMixCtx * kOrders; i += blockDim.x) s.w[i] = init->w[(i & ~7) + dec_order(i & 7)];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4096; i += blockDim.x) tab->squash[i] += tab->squash[i] < 2048;  // see dec_mix
+  __syncthreads();
+  return tab;
+}
+
+// Warp = chunk (tasks handed out by a queue): a nibble per round, the next
+// round's gathers issued as soon as one is decoded.
 __global__ void __launch_bounds__(kFixedDecWarps * 32)
     fixed_decode_kernel(const FixedTask *tasks, uint32_t ntasks, const uint8_t *image, const ModelInit *init,
                         uint32_t *queue) {
-  __shared__ FixedSmem f;
-  __shared__ __align__(16) uint8_t wins[kFixedDecWarps][kDecWin];
-  fixed_load_model(&f, init);
-  __syncthreads();
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  DecSmem s;
+  const Tables *tab = fixed_dec_load(smem_raw, image, init, s);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint8_t *win = wins[warp];
-  const int node = lane % kDecNodes;
-  const int depth = 31 - __clz(node + 1);
-  const uint32_t pbits = (uint32_t)(node + 1 - (1 << depth));
+  uint8_t *win = smem_raw + kFixedDecWin + warp * kDecWin;
+  const DecLane<true> ln(s, image, lane);
   for (;;) {
     uint32_t ti = 0;
     if (lane == 0) ti = atomicAdd(queue, 1u);
     ti = __shfl_sync(0xffffffffu, ti, 0);
     if (ti >= ntasks) break;
     const FixedTask t = tasks[ti];
-    const uint8_t *pay = t.in;
-    const uint64_t plen = t.in_len;
-    long long wbase = dec_refill(win, pay, plen, 0, lane);
-    uint32_t x1 = 0, x2 = 0xffffffffu, x = 0;
-    uint64_t ioff = 0;
-    for (int i = 0; i < 4; i++, ioff++) x = (x << 8) | (ioff < plen ? (uint32_t)win[(long long)ioff - wbase] : 255u);
+    DecCoder c;
+    dec_open(c, win, t.in, t.in_len, lane);
     uint32_t hist[7] = {0, 0, 0, 0, 0, 0, 0};
-    uint32_t cur = 0;
+    uint32_t cur = 0, kk[4], st[4];
     int r = 0;
-    uint32_t st[kOrders];
-    auto gather = [&]() {
-      const uint32_t h0 = (1u << (r + depth)) | (cur << depth) | pbits;
-      BitKeys kk;
-      bit_keys(h0, hist, kk);
-CUCM_UNROLL
-      for (int o = 0; o < kOrders; o++) st[o] = fixed_state(image, o, kk.k[o]);
-    };
     const uint64_t rounds = 2 * t.out_cap;
-    if (rounds) gather();
+    if (rounds) ln.gather(cur, r, hist, kk, st);
+    uint32_t next = dec_ahead(c, win, t.in, t.in_len, lane);
     for (uint64_t rd = 0; rd < rounds; rd++) {
-      if ((long long)ioff + 16 > wbase + kDecWin) wbase = dec_refill(win, pay, plen, ioff, lane);
-      int smp[kOrders];
-CUCM_UNROLL
-      for (int o = 0; o < kOrders; o++) smp[o] = f.spf[st[o] * kOrders + o];
-      const uint32_t f_node = (uint32_t)fixed_mix(&f, smp, (int)hist[0]) << 20;
-      int n = 0;
-      uint32_t nib = 0;
-      uint32_t fv = __shfl_sync(0xffffffffu, f_node, 0);
-CUCM_UNROLL
-      for (int i = 0; i < 4; i++) {
-        uint32_t fa = 0, fb = 0;
-        if (i < 3) {
-          fa = __shfl_sync(0xffffffffu, f_node, 2 * n + 1);
-          fb = __shfl_sync(0xffffffffu, f_node, 2 * n + 2);
-        }
-        const uint32_t xm = x1 + __umulhi(x2 - x1, fv);
-        const int y = x <= xm;
-        if (y) x2 = xm; else x1 = xm + 1;
-        while ((x1 ^ x2) < 0x1000000u) {
-          x1 <<= 8;
-          x2 = (x2 << 8) | 255u;
-          x = (x << 8) | (ioff < plen ? (uint32_t)win[(long long)ioff - wbase] : 255u);
-          ioff++;
-        }
-        nib = (nib << 1) | (uint32_t)y;
-        n = 2 * n + 1 + y;
-        fv = y ? fb : fa;
-      }
+      int smp[4], cxt;
+      const uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+      DecPath path;
+      const uint32_t nib = dec_nibble(c, path, pr << 20, next, win, lane);
       cur = (cur << 4) | nib;
       r += 4;
       if (r == 8) {
         if (lane == 0) t.out[rd >> 1] = (uint8_t)cur;
-CUCM_UNROLL
-        for (int i = 6; i > 0; i--) hist[i] = hist[i - 1];
-        hist[0] = cur;
+        dec_push(hist, cur);
         cur = 0;
         r = 0;
       }
-      if (rd + 1 < rounds) gather();
+      if (rd + 1 < rounds) ln.gather(cur, r, hist, kk, st);
+      dec_settle(c, path, win);
+      next = dec_ahead(c, win, t.in, t.in_len, lane);
     }
     __syncwarp();
+  }
+}
+
+// CTA = chunk: a byte per round, the second nibble's nodes gathered with the
+// first one's by a warp for each likely first nibble (decompress_wide.cuh, with
+// nothing to update or record).
+constexpr int kFixedWideThreads = 32 * (1 + kWideGuess);
+
+__global__ void __launch_bounds__(kFixedWideThreads, 1)
+    fixed_decode_wide_kernel(const FixedTask *tasks, uint32_t ntasks, const uint8_t *image, const ModelInit *init,
+                             uint32_t *queue) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  __shared__ WideSmem ws;
+  __shared__ uint32_t s_task;
+  DecSmem s;
+  const Tables *tab = fixed_dec_load(smem_raw, image, init, s);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint8_t *win = smem_raw + kFixedDecWin;
+  const DecLane<true> ln(s, image, lane);
+  volatile uint32_t *ready = ws.ready;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) s_task = atomicAdd(queue, 1u);
+    if (tid < kWideGuess) ws.ready[tid] = 0;
+    __syncthreads();
+    const uint32_t ti = s_task;
+    if (ti >= ntasks) break;
+    const FixedTask t = tasks[ti];
+    uint32_t hist[7] = {0, 0, 0, 0, 0, 0, 0};
+    uint32_t kk[4], st[4];
+    int smp[4], cxt;
+    if (warp == 0) {
+      DecCoder c;
+      dec_open(c, win, t.in, t.in_len, lane);
+      if (t.out_cap) ln.gather(0, 0, hist, kk, st);
+      uint32_t next = dec_ahead(c, win, t.in, t.in_len, lane);
+      for (uint64_t b = 0; b < t.out_cap; b++) {
+        const uint32_t seq = 2 * (uint32_t)b;
+        uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+        DecPath path;
+        const uint32_t hi = dec_nibble(c, path, pr << 20, next, win, lane);
+        dec_settle(c, path, win);
+        next = dec_ahead(c, win, t.in, t.in_len, lane);
+        // its warp came through the last crossing, so this ends with its
+        // gathers (past the bound the nibble is predicted here, with the same
+        // result)
+        uint32_t spins = 0, have;
+        while ((have = ready[hi]) != seq + 1 && have != seq + 2)
+          if (++spins >= kDecSpinLimit) break;
+        __threadfence_block();
+        uint32_t f_node = ws.f[hi][lane & 15];
+        if (have != seq + 1) {
+          ln.gather(hi, 4, hist, kk, st);
+          pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+          f_node = pr << 20;
+        }
+        const uint32_t lo = dec_nibble(c, path, f_node, next, win, lane);
+        const uint32_t byte = (hi << 4) | lo;
+        if (lane == 0) ws.byte[b & 1] = byte;
+        __syncwarp();
+        if (spins < kDecSpinLimit)
+          wide_byte_arrive();
+        else
+          wide_byte_wait();
+        dec_push(hist, byte);
+        if (b + 1 < t.out_cap) ln.gather(0, 0, hist, kk, st);
+        dec_settle(c, path, win);
+        next = dec_ahead(c, win, t.in, t.in_len, lane);
+        if (lane == 0) t.out[b] = (uint8_t)byte;
+      }
+    } else {
+      const uint32_t guess = (uint32_t)(warp - 1);
+      for (uint64_t b = 0; b < t.out_cap; b++) {
+        const bool follow = wide_follow(s, tab, guess, hist[0], lane);
+        if (follow) {
+          ln.gather(guess, 4, hist, kk, st);
+          const uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+          if (lane < kDecNodes) ws.f[guess][lane] = pr << 20;
+        }
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence_block();
+          ready[guess] = 2 * (uint32_t)b + (follow ? 1 : 2);
+        }
+        wide_byte_wait();
+        dec_push(hist, ws.byte[b & 1]);
+      }
+    }
   }
 }
