@@ -95,7 +95,7 @@ cudaError_t launch_decompress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t
 
 // Fixed-model variant: coder inputs of every byte of every task (first[]:
 // prefix sums of the chunk lengths, total bytes), then one coder thread per
-// task; and the decoder, one warp per task from a zeroed queue counter.
+// task; and the decoder, one warp or CTA per task from a zeroed queue counter.
 // image / d_init: the prelearned model in the device layout.
 cudaError_t launch_fixed_encode(const FixedTask *d_tasks, const uint64_t *d_first, uint32_t ntasks, uint64_t total,
                                 const uint8_t *image, const ModelInit *d_init, uint32_t *d_status, int sm_count,
