@@ -91,7 +91,7 @@ typedef struct cucm_tuning {
                         * flight, else pairs spread over all SMs first */
   int dec_tables;      /* decoder order 0/1 tables: 0 = shared memory where it fits, 1 = slot tables */
   int cmp_ctas;        /* pipelined compressor CTAs (chunks) per SM, 1 or 2; 0 = most that fit */
-  uint32_t dec_spin_limit; /* polls bounding the decoder's wait between its two warps; 0 = 2^27 (seconds).
+  uint32_t dec_spin_limit; /* polls bounding the decoder's waits between its warps; 0 = 2^27 (seconds).
                             * When a wait runs out the call returns CUCM_ETIMEOUT and the context stays
                             * usable; a small value makes that happen on purpose (tests). */
 } cucm_tuning;
