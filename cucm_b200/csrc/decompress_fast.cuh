@@ -11,8 +11,8 @@
 //   * gives the 15 nodes of the nibble's speculation tree (every prefix of
 //     0..3 bits) their 8 context keys and frozen slot states -- two lanes per
 //     node, the even and the odd orders, the 6 hashed orders' gathers in
-//     flight together (orders 0 and 1 come from shared memory when the CTA has
-//     room for them), so a round costs one memory round trip;
+//     flight together (orders 0 and 1 come from shared memory for a chunk alone
+//     in its CTA), so a round costs one memory round trip;
 //   * mixes and squashes each node's prediction against the frozen model
 //     (probabilities kept stretched) and decodes the 4 bits, a lane per leaf of
 //     the tree (dec_nibble);

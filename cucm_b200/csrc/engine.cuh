@@ -71,7 +71,7 @@ struct EngineConfig {
   bool generic = false;        // force the generic (non-pipelined) kernels
   int sm_count = 0;            // SMs of the device (0 = query)
   int dec_pairs = 0;           // decoder chunks per CTA (0 = spread over all SMs first)
-  int dec_tables = 0;          // decoder order 0/1 tables: 0 = shared memory where it fits, 1 = slot tables
+  int dec_tables = 0;          // decoder order 0/1 tables: 0 = shared memory where it pays, 1 = slot tables
   int cmp_ctas = 0;            // pipelined compressor CTAs per SM (0 = derived)
   uint32_t others = 0;         // decoder: chunks that other launches may have in flight beside this one's
   uint32_t spin_limit = 0;     // decoder: polls bounding the wait for a published round (0 = default)

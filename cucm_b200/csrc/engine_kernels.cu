@@ -717,10 +717,11 @@ cudaError_t launch_decompress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t
     if (cfg.dec_pairs > 0) wpc = cfg.dec_pairs;
     if (wpc > wmax) wpc = wmax;
     if (wpc < 1) wpc = 1;
-    // up to two chunks per CTA leave room for their order 0/1 tables in
-    // shared memory
+    // a chunk alone in its CTA keeps its order 0/1 tables in shared memory
+    // (two would fit, but a fourth gather costs less than their lookups take
+    // from the load/store pipe: 64 MiB in 256 chunks, 722 ms from HBM, 731)
     const DecLayout Low = make_dec_layout(unit, wpc, true);
-    const bool low = cfg.dec_tables == 0 && wpc <= 2 && Low.total <= kDecSmemLimit;
+    const bool low = cfg.dec_tables == 0 && wpc == 1 && Low.total <= kDecSmemLimit;
     const DecLayout L = low ? Low : make_dec_layout(unit, wpc);
     const void *kern = low ? (const void *)decompress_pair_kernel<true> : (const void *)decompress_pair_kernel<false>;
     cudaError_t e = set_smem(kern, L.total);
