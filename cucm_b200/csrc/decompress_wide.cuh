@@ -44,20 +44,16 @@ constexpr float kWideLeast = 0.065f;
 struct WideSmem {
   uint32_t f[kWideGuess][kDecNodes + 1];  // predictions << 20 of the nodes below each first nibble
   uint32_t ready[kWideGuess];             // 2 * byte + 1 when they are there, 2 * byte + 2 when not followed
-  uint32_t byte[2];                       // the byte decoded last, by byte parity
+  uint32_t byte[kWidePlaces];             // the last bytes decoded, byte n in place n % kWidePlaces
 };
 
-// Named barrier 1 (0 is the CTA's): a byte is known.  The decoding warp arrives
-// and goes on, the guessing warps wait.  It never arrives twice at one
-// crossing: before it arrives again it has seen a `ready` of the next byte,
-// whose writer came through this crossing with all the others.  For the same
-// reason two bytes' places are enough for `byte`.  Where its wait for that
-// `ready` has run out, it crosses with the guessing warps instead.
-__device__ __forceinline__ void wide_byte_arrive() {
-  asm volatile("bar.arrive 1, %0;" ::"n"(32 * (1 + kWideGuess)) : "memory");
+// Byte nth is known (wide_crossing.h): the decoding warp arrives and goes on, or
+// waits too where its wait for a `ready` has run out.
+__device__ __forceinline__ void wide_byte_arrive(uint32_t nth) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1 + nth % kWideBarriers), "n"(32 * (1 + kWideGuess)) : "memory");
 }
-__device__ __forceinline__ void wide_byte_wait() {
-  asm volatile("bar.sync 1, %0;" ::"n"(32 * (1 + kWideGuess)) : "memory");
+__device__ __forceinline__ void wide_byte_wait(uint32_t nth) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + nth % kWideBarriers), "n"(32 * (1 + kWideGuess)) : "memory");
 }
 
 // Whether first nibble `guess` after byte c1 is likely enough, by the order-1
@@ -137,12 +133,12 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
         const uint32_t lo = dec_nibble(c, path, f_node, next, s.win, lane);
         if (have != seq + 1) dec_write_record(s, ln, dec_record(ln, kk, st, smp, pr, cxt, lo), 2 * b + 1);
         const uint32_t byte = (hi << 4) | lo;
-        if (lane == 0) ws.byte[nth & 1] = byte;
+        if (lane == 0) ws.byte[nth % kWidePlaces] = byte;
         __syncwarp();
         if (ok)
-          wide_byte_arrive();
+          wide_byte_arrive(nth);
         else
-          wide_byte_wait();
+          wide_byte_wait(nth);
         dec_push(hist, byte);
         if (b + 1 < nb) ln.gather(0, 0, hist, kk, st);
         dec_settle(c, path, s.win);
@@ -171,8 +167,8 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
           __threadfence_block();
           ready[guess] = seq + (follow ? 1 : 2);
         }
-        wide_byte_wait();
-        const uint32_t byte = ws.byte[nth & 1];
+        wide_byte_wait(nth);
+        const uint32_t byte = ws.byte[nth % kWidePlaces];
         if ((byte >> 4) == guess) {
           // the warp of the nibble that came records its path (the decoding warp
           // has, where it was not followed) and says so: the word only grows, since

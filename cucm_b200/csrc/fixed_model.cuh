@@ -272,9 +272,8 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
         const uint32_t hi = dec_nibble(c, path, pr << 20, next, win, lane);
         dec_settle(c, path, win);
         next = dec_ahead(c, win, t.in, t.in_len, lane);
-        // its warp came through the last crossing, so this ends with its
-        // gathers (past the bound the nibble is predicted here, with the same
-        // result)
+        // ends with its warp's gathers; past the bound the nibble is predicted
+        // here, with the same result, so there is nothing to report
         uint32_t spins = 0, have;
         while ((have = ready[hi]) != seq + 1 && have != seq + 2)
           if (++spins >= kDecSpinLimit) break;
@@ -287,12 +286,12 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
         }
         const uint32_t lo = dec_nibble(c, path, f_node, next, win, lane);
         const uint32_t byte = (hi << 4) | lo;
-        if (lane == 0) ws.byte[b & 1] = byte;
+        if (lane == 0) ws.byte[b % kWidePlaces] = byte;
         __syncwarp();
         if (spins < kDecSpinLimit)
-          wide_byte_arrive();
+          wide_byte_arrive((uint32_t)b);
         else
-          wide_byte_wait();
+          wide_byte_wait((uint32_t)b);
         dec_push(hist, byte);
         if (b + 1 < t.out_cap) ln.gather(0, 0, hist, kk, st);
         dec_settle(c, path, win);
@@ -313,8 +312,8 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
           __threadfence_block();
           ready[guess] = 2 * (uint32_t)b + (follow ? 1 : 2);
         }
-        wide_byte_wait();
-        dec_push(hist, ws.byte[b & 1]);
+        wide_byte_wait((uint32_t)b);
+        dec_push(hist, ws.byte[b % kWidePlaces]);
       }
     }
   }
