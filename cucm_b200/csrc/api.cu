@@ -498,7 +498,7 @@ int encode_fixed(cucm_ctx *c, const std::vector<Seg> &segs, uint64_t cs, const M
   return CUCM_OK;
 }
 
-// Decode every chunk of fixed-model containers: one warp per chunk.
+// Decode every chunk of fixed-model containers: a CTA or a warp per chunk.
 int decode_fixed(cucm_ctx *c, const std::vector<DecJob> &jobs, const ModelSource &ms) {
   std::vector<FixedTask> tasks;
   for (const DecJob &j : jobs)

@@ -143,6 +143,13 @@ __device__ __forceinline__ uint32_t ld_slot_state(const uint8_t *p) {
   asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+// One from tables that are never written: through L1, where chunks that read
+// the same tables find each other's lines.
+__device__ __forceinline__ uint32_t ld_kept_state(const uint8_t *p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // Warp-wide refill of the payload window so that it starts at or just below
 // payload byte `at`, on a 16-byte boundary of the payload's address (so the
@@ -473,8 +480,8 @@ __device__ __forceinline__ uint32_t dec_mix(const int32_t *w, int cxt, const int
 // A lane of a warp that predicts the nodes of a speculation tree.  Each half
 // warp holds the 15 nodes (its last lane doubles the last one), the lower half
 // their even orders, the upper half the odd ones, so that a round takes three
-// gather instructions of 30 lines.
-template <bool kLow>
+// gather instructions of 30 lines.  kKept: the slot tables are read only.
+template <bool kLow, bool kKept = false>
 struct DecLane {
   int half, depth;
   uint32_t pbits;
@@ -506,13 +513,16 @@ CUCM_UNROLL
     for (int q = 0; q < 4; q++) kk[q] = half ? k.k[2 * q + 1] : k.k[2 * q];
     if (kLow) st[0] = low[kk[0]];
 CUCM_UNROLL
-    for (int q = 0; q < 3; q++) st[q + 1] = ld_slot_state(tables[q] + kk[q + 1]);
-    if (!kLow) st[0] = ld_slot_state(low + kk[0]);
+    for (int q = 0; q < 3; q++) st[q + 1] = state(tables[q] + kk[q + 1]);
+    if (!kLow) st[0] = state(low + kk[0]);
+  }
+  static __device__ __forceinline__ uint32_t state(const uint8_t *p) {
+    return kKept ? ld_kept_state(p) : ld_slot_state(p);
   }
 
   // Stretch, mixer context, mixer output (cucm_decompress_v2.cu:774-809).
-  __device__ __forceinline__ uint32_t predict(const DecSmem &s, const Tables *tab, const uint32_t st[4], uint32_t c1,
-                                              int smp[4], int &cxt) const {
+  __device__ __forceinline__ uint32_t predict(const DecSmem &s, const uint16_t *squash, const uint32_t st[4],
+                                              uint32_t c1, int smp[4], int &cxt) const {
     int olen = 0;
 CUCM_UNROLL
     for (int q = 0; q < 4; q++) smp[q] = spf[q * kDecSpfRow + st[q]];
@@ -520,7 +530,7 @@ CUCM_UNROLL
     for (int q = 0; q < 4; q++) olen += (smp[q] != 1);
     olen += __shfl_xor_sync(0xffffffffu, olen, 16);
     cxt = olen + (int)(c1 >> 5) * 10;
-    return dec_mix(s.w, cxt, smp, half, tab->squash);
+    return dec_mix(s.w, cxt, smp, half, squash);
   }
 };
 
@@ -673,7 +683,7 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
     uint32_t next = dec_ahead(c, s.win, pay, plen, lane);
     for (int rd = 0; rd < nr; rd++) {
       int smp[4], cxt;
-      const uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+      const uint32_t pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
       DecPath path;
       const uint32_t nib = dec_nibble(c, path, pr << 20, next, s.win, lane);
       const DecRecord rec = dec_record(ln, kk, st, smp, pr, cxt, nib);

@@ -109,7 +109,7 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
       for (int b = 0; b < nb; b++) {
         const uint32_t nth = bytes + (uint32_t)b, seq = 2 * nth;
         int smp[4], cxt;
-        uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+        uint32_t pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
         DecPath path;
         const uint32_t hi = dec_nibble(c, path, pr << 20, next, s.win, lane);
         const DecRecord first = dec_record(ln, kk, st, smp, pr, cxt, hi);
@@ -127,7 +127,7 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
         uint32_t f_node = ws.f[hi][lane & 15];
         if (have != seq + 1) {  // not followed, and there it is
           ln.gather(hi, 4, hist, kk, st);
-          pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+          pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
           f_node = pr << 20;
         }
         const uint32_t lo = dec_nibble(c, path, f_node, next, s.win, lane);
@@ -159,7 +159,7 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
         uint32_t pr = 0;
         if (follow) {
           ln.gather(guess, 4, hist, kk, st);
-          pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+          pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
           if (lane < kDecNodes) ws.f[guess][lane] = pr << 20;
         }
         __syncwarp();

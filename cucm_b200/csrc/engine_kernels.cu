@@ -600,7 +600,7 @@ cudaError_t launch_fixed_decode(const FixedTask *d_tasks, uint32_t ntasks, const
   // 37.0 -> 24.8 ms with 16 chunks, 36.8 -> 26.5 with 148 (random bytes 37.6 ->
   // 35.9); two waves of CTAs would not pay.
   if (ntasks <= sms) {
-    const size_t smem = fixed_dec_smem_bytes(1);
+    const size_t smem = kFixedWideSmem;
     cudaError_t e = set_smem((const void *)fixed_decode_wide_kernel, smem);
     if (e != cudaSuccess) return e;
     fixed_decode_wide_kernel<<<ntasks, kFixedWideThreads, smem, stream>>>(d_tasks, ntasks, image, d_init, d_queue);
@@ -614,7 +614,7 @@ cudaError_t launch_fixed_decode(const FixedTask *d_tasks, uint32_t ntasks, const
   const size_t smem = fixed_dec_smem_bytes((int)warps);
   cudaError_t e = set_smem((const void *)fixed_decode_kernel, smem);
   if (e != cudaSuccess) return e;
-  fixed_decode_kernel<<<std::min(want, sms * 2), warps * 32, smem, stream>>>(d_tasks, ntasks, image, d_init, d_queue);
+  fixed_decode_kernel<<<std::min(want, sms * 4), warps * 32, smem, stream>>>(d_tasks, ntasks, image, d_init, d_queue);
   return cudaGetLastError();
 }
 

@@ -159,44 +159,44 @@ CUCM_UNROLL
   if (base > t.out_cap) atomicOr(status, (uint32_t)kDevOverflow);
 }
 
-// The decoders.  The model is only read, so its order 0 and 1 tables, stretched
-// probabilities and weights sit in shared memory once per CTA, in the layout of
-// the adaptive decoder, whose lanes (DecLane) and coder (dec_nibble) these use.
+// The decoders.  They use the adaptive decoder's lanes (DecLane) and coder
+// (dec_nibble), so the model's stretched probabilities and weights sit in its
+// layout in shared memory, once per CTA.
 constexpr int kFixedDecWarps = 8;
-constexpr size_t kFixedDecSpf = kHashedOff, kFixedDecW = kFixedDecSpf + sizeof(int16_t) * kOrders * kDecSpfRow,
-                 kFixedDecTab = kFixedDecW + sizeof(int32_t) * kMixCtx * kOrders,
-                 kFixedDecWin = kFixedDecTab + sizeof(Tables);
-inline size_t fixed_dec_smem_bytes(int windows) { return kFixedDecWin + (size_t)windows * kDecWin; }
 
-__device__ __forceinline__ Tables *fixed_dec_load(uint8_t *smem, const uint8_t *image, const ModelInit *init,
-                                                  DecSmem &s) {
-  s.t01 = smem;
-  s.spf = reinterpret_cast<int16_t *>(smem + kFixedDecSpf);
-  s.w = reinterpret_cast<int32_t *>(smem + kFixedDecW);
-  Tables *tab = reinterpret_cast<Tables *>(smem + kFixedDecTab);
-  copy_tables(&g_tables, tab);
-  const uint4 *src = reinterpret_cast<const uint4 *>(image);
-  for (int i = threadIdx.x; i < (int)(kHashedOff / 16); i += blockDim.x) reinterpret_cast<uint4 *>(s.t01)[i] = src[i];
+// The model but its slot tables, in shared memory behind `kept`.
+constexpr size_t kFixedDecSpf = sizeof(int16_t) * kOrders * kDecSpfRow, kFixedDecW = sizeof(int32_t) * kMixCtx * kOrders;
+__device__ __forceinline__ void fixed_dec_model(uint8_t *kept, const ModelInit *init, DecSmem &s) {
+  s.spf = reinterpret_cast<int16_t *>(kept);
+  s.w = reinterpret_cast<int32_t *>(kept + kFixedDecSpf);
   for (int i = threadIdx.x; i < 256 * kOrders; i += blockDim.x)
     s.spf[(i >> 8) * kDecSpfRow + (i & 255)] = g_tables.stretch[init->statep[dec_order(i >> 8)][i & 255] >> 20];
   for (int i = threadIdx.x; i < kMixCtx * kOrders; i += blockDim.x) s.w[i] = init->w[(i & ~7) + dec_order(i & 7)];
-  __syncthreads();
-  for (int i = threadIdx.x; i < 4096; i += blockDim.x) tab->squash[i] += tab->squash[i] < 2048;  // see dec_mix
-  __syncthreads();
-  return tab;
 }
 
 // Warp = chunk (tasks handed out by a queue): a nibble per round, the next
-// round's gathers issued as soon as one is decoded.
-__global__ void __launch_bounds__(kFixedDecWarps * 32)
+// round's gathers issued as soon as one is decoded.  All chunks read the same
+// tables, so the gathers go through L1 and everything else is kept small: 31 KB
+// a CTA, four CTAs an SM, 100 KB of L1 beside them.  Text in chunks of 2 KiB,
+// ms against order 0/1 tables in shared memory, gathers past L1 and two CTAs an
+// SM: 149 chunks 4.5 and 4.5, 500 4.6 and 5.2, 1,184 5.5 and 10.1, 2,368 9.0 and
+// 20.1, 4,736 18.8 and 40.1.
+constexpr size_t kFixedDecSquash = kFixedDecSpf + kFixedDecW, kFixedDecWin = kFixedDecSquash + sizeof(uint16_t) * 4096;
+inline size_t fixed_dec_smem_bytes(int warps) { return kFixedDecWin + (size_t)warps * kDecWin; }
+
+__global__ void __launch_bounds__(kFixedDecWarps * 32, 4)
     fixed_decode_kernel(const FixedTask *tasks, uint32_t ntasks, const uint8_t *image, const ModelInit *init,
                         uint32_t *queue) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   DecSmem s;
-  const Tables *tab = fixed_dec_load(smem_raw, image, init, s);
+  fixed_dec_model(smem_raw, init, s);
+  uint16_t *squash = reinterpret_cast<uint16_t *>(smem_raw + kFixedDecSquash);
+  for (int i = threadIdx.x; i < 4096; i += blockDim.x)  // see dec_mix
+    squash[i] = g_tables.squash[i] + (g_tables.squash[i] < 2048);
+  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint8_t *win = smem_raw + kFixedDecWin + warp * kDecWin;
-  const DecLane<true> ln(s, image, lane);
+  const DecLane<false, true> ln(s, image, lane);
   for (;;) {
     uint32_t ti = 0;
     if (lane == 0) ti = atomicAdd(queue, 1u);
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kFixedDecWarps * 32)
     uint32_t next = dec_ahead(c, win, t.in, t.in_len, lane);
     for (uint64_t rd = 0; rd < rounds; rd++) {
       int smp[4], cxt;
-      const uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+      const uint32_t pr = ln.predict(s, squash, st, hist[0], smp, cxt);
       DecPath path;
       const uint32_t nib = dec_nibble(c, path, pr << 20, next, win, lane);
       cur = (cur << 4) | nib;
@@ -236,6 +236,8 @@ __global__ void __launch_bounds__(kFixedDecWarps * 32)
 // first one's by a warp for each likely first nibble (decompress_wide.cuh, with
 // nothing to update or record).
 constexpr int kFixedWideThreads = 32 * (1 + kWideGuess);
+constexpr size_t kFixedWideTab = kHashedOff, kFixedWideKept = kFixedWideTab + sizeof(Tables),
+                 kFixedWideWin = kFixedWideKept + kFixedDecSpf + kFixedDecW, kFixedWideSmem = kFixedWideWin + kDecWin;
 
 __global__ void __launch_bounds__(kFixedWideThreads, 1)
     fixed_decode_wide_kernel(const FixedTask *tasks, uint32_t ntasks, const uint8_t *image, const ModelInit *init,
@@ -244,9 +246,16 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
   __shared__ WideSmem ws;
   __shared__ uint32_t s_task;
   DecSmem s;
-  const Tables *tab = fixed_dec_load(smem_raw, image, init, s);
+  s.t01 = smem_raw;
+  Tables *tab = reinterpret_cast<Tables *>(smem_raw + kFixedWideTab);
+  copy_tables(&g_tables, tab);
+  const uint4 *src = reinterpret_cast<const uint4 *>(image);
+  for (int i = threadIdx.x; i < (int)(kHashedOff / 16); i += blockDim.x) reinterpret_cast<uint4 *>(s.t01)[i] = src[i];
+  fixed_dec_model(smem_raw + kFixedWideKept, init, s);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4096; i += blockDim.x) tab->squash[i] += tab->squash[i] < 2048;  // see dec_mix
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint8_t *win = smem_raw + kFixedDecWin;
+  uint8_t *win = smem_raw + kFixedWideWin;
   const DecLane<true> ln(s, image, lane);
   volatile uint32_t *ready = ws.ready;
   for (;;) {
@@ -267,7 +276,7 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
       uint32_t next = dec_ahead(c, win, t.in, t.in_len, lane);
       for (uint64_t b = 0; b < t.out_cap; b++) {
         const uint32_t seq = 2 * (uint32_t)b;
-        uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+        uint32_t pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
         DecPath path;
         const uint32_t hi = dec_nibble(c, path, pr << 20, next, win, lane);
         dec_settle(c, path, win);
@@ -281,7 +290,7 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
         uint32_t f_node = ws.f[hi][lane & 15];
         if (have != seq + 1) {
           ln.gather(hi, 4, hist, kk, st);
-          pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+          pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
           f_node = pr << 20;
         }
         const uint32_t lo = dec_nibble(c, path, f_node, next, win, lane);
@@ -304,7 +313,7 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
         const bool follow = wide_follow(s, tab, guess, hist[0], lane);
         if (follow) {
           ln.gather(guess, 4, hist, kk, st);
-          const uint32_t pr = ln.predict(s, tab, st, hist[0], smp, cxt);
+          const uint32_t pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
           if (lane < kDecNodes) ws.f[guess][lane] = pr << 20;
         }
         __syncwarp();
