@@ -284,18 +284,6 @@ __device__ __forceinline__ void dec_settle(DecCoder &c, const DecPath &w, const 
   }
 }
 
-// `if (mine) *at = v`, in program order with the other such stores of the
-// warp: where lanes share an address, the last one's value stays.
-__device__ __forceinline__ void store_turn8(bool mine, uint32_t at, uint32_t v) {
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.u8 [%1], %2; }" ::"r"((uint32_t)mine), "r"(at), "r"(v)
-               : "memory");
-}
-__device__ __forceinline__ void store_turn32(bool mine, uint32_t at, uint32_t v) {
-  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.u32 [%1], %2; }" ::"r"((uint32_t)mine), "r"(at),
-               "r"(v)
-               : "memory");
-}
-
 // Model update of one round's 4 bits (lane = column lane & 7, bit lane >> 3):
 // the live state of each slot (what an earlier bit of the unit left there, else
 // the frozen state the prediction saw), its next state, the StateMap
@@ -352,17 +340,19 @@ __device__ __forceinline__ void dec_update_round(const DecSmem &s, const Tables 
   const uint32_t next = tab->nex[live][y];
   uint32_t v = s.spl[o * kDecSplRow + live];
   // positions of this round with the same hash
-  const uint32_t h1 = __shfl_up_sync(0xffffffffu, h, 8), h2 = __shfl_up_sync(0xffffffffu, h, 16),
-                 h3 = __shfl_up_sync(0xffffffffu, h, 24);
+  const uint32_t h0 = __shfl_sync(0xffffffffu, h, o), h1 = __shfl_sync(0xffffffffu, h, o + 8),
+                 h2 = __shfl_sync(0xffffffffu, h, o + 16), h3 = __shfl_sync(0xffffffffu, h, o + 24);
   uint32_t before = p < base ? p : kDecNone;
-  if (i >= 3 && h3 == h) before = j - 3;
-  if (i >= 2 && h2 == h) before = j - 2;
-  if (i >= 1 && h1 == h) before = j - 1;
+  if (i > 0 && h0 == h) before = base;
+  if (i > 1 && h1 == h) before = base + 1;
+  if (i > 2 && h2 == h) before = base + 2;
+  const bool last_of_hash = !((i < 1 && h1 == h) || (i < 2 && h2 == h) || (i < 3 && h3 == h));
   // a state met m times earlier in the round has count min(count + m, 1023)
   const uint32_t l0 = __shfl_sync(0xffffffffu, live, o), l1 = __shfl_sync(0xffffffffu, live, o + 8),
-                 l2 = __shfl_sync(0xffffffffu, live, o + 16);
+                 l2 = __shfl_sync(0xffffffffu, live, o + 16), l3 = __shfl_sync(0xffffffffu, live, o + 24);
   const bool e0 = i > 0 && l0 == live, e1 = i > 1 && l1 == live, e2 = i > 2 && l2 == live;
   const uint32_t m = (uint32_t)e0 + (uint32_t)e1 + (uint32_t)e2;
+  const bool last_of_state = !((i < 1 && l1 == live) || (i < 2 && l2 == live) || (i < 3 && l3 == live));
   const uint32_t rate = tab->dt[min((v & 1023u) + m, 1023u)];
   uint32_t nv = statep_next(v, y, rate);
   if (__any_sync(0xffffffffu, m != 0)) {
@@ -376,17 +366,13 @@ __device__ __forceinline__ void dec_update_round(const DecSmem &s, const Tables 
     v = e2 ? n2 : v;
     nv = statep_next(v, y, rate);
   }
-  // writes; where bits share a place, the later bit's stays
+  __syncwarp();  // everything is read
+  // writes; where bits share a place, the last of them writes
   if (again) s.rk[found * kOrders + o] = k | 0x80000000u;
   s.ons[r] = (uint8_t)next;
   s.och[r] = (uint8_t)before;
-  const uint32_t at = (uint32_t)__cvta_generic_to_shared(last);
-  const uint32_t sp = (uint32_t)__cvta_generic_to_shared(s.spl + o * kDecSplRow + live);
-CUCM_UNROLL
-  for (int t = 0; t < 4; t++) {
-    store_turn8(i == t, at, j);
-    store_turn32(i == t, sp, nv);
-  }
+  if (last_of_hash) *last = (uint8_t)j;
+  if (last_of_state) s.spl[o * kDecSplRow + live] = nv;
   atomicAdd(&s.dw[cx * kOrders + o], delta);
   __syncwarp();
 }
