@@ -24,6 +24,7 @@
 
 #include "../../include/cucm.h"
 #include "engine.cuh"
+#include "framing_window.h"
 #include "host_model.h"
 #include "model.cuh"
 
@@ -809,8 +810,6 @@ int cucm_compress_dev(cucm_ctx *c, const uint8_t *in, uint64_t n, const cucm_par
   return compress_containers(c, 1, &in, &n, p, &out, &cap, out_n, &st, true);
 }
 
-constexpr uint64_t kFramingHead = 4096;
-
 // Decompress `count` containers (decompress, cucm_decompress_v2.cu:1185-1248,
 // per container).  Containers without a prelearn prefix are decoded in one
 // engine run per unit length; a prelearn prefix means its own model and run.
@@ -821,7 +820,8 @@ static int decompress_containers(cucm_ctx *c, uint32_t count, const uint8_t *con
   // The header, prelearn block and batch framing are parsed on the host.  Of a
   // container in device memory only those are fetched: its first bytes, which
   // mostly hold all of them, then what lies further on.  (The whole of it, by
-  // way of pageable memory, took 26 ms of a 811 ms call over 64 MiB.)
+  // way of pageable memory, took 26 ms of a 811 ms call over 64 MiB; see
+  // framing_window.h for short batches.)
   std::vector<std::vector<uint8_t>> host_copy(dev ? count : 0);
   std::vector<const uint8_t *> h(count);
   std::vector<Parsed> ph(count);
@@ -833,7 +833,7 @@ static int decompress_containers(cucm_ctx *c, uint32_t count, const uint8_t *con
     if (status[i]) continue;
     h[i] = ins[i];
     if (dev) {
-      host_copy[i].resize(std::min<uint64_t>(ns[i], kFramingHead));
+      host_copy[i].resize(std::min<uint64_t>(ns[i], kFramingPiece));
       CK(cudaMemcpy(host_copy[i].data(), ins[i], host_copy[i].size(), cudaMemcpyDeviceToHost));
       h[i] = host_copy[i].data();
     }
@@ -853,15 +853,19 @@ static int decompress_containers(cucm_ctx *c, uint32_t count, const uint8_t *con
       CK(cudaMemcpy(host_copy[i].data() + have, ins[i] + have, body_off - have, cudaMemcpyDeviceToHost));
       h[i] = host_copy[i].data();
     }
-    std::vector<uint8_t> piece;
-    auto read = [&](uint64_t at, uint64_t bytes) -> const uint8_t * {
+    cudaError_t fetched = cudaSuccess;
+    auto fetch = [&](uint64_t at, uint64_t bytes, uint8_t *to) {
+      fetched = cudaMemcpy(to, ins[i] + at, bytes, cudaMemcpyDeviceToHost);
+      return fetched == cudaSuccess;
+    };
+    const uint64_t held = dev ? host_copy[i].size() : ns[i];
+    FramingWindow<decltype(fetch)> window(fetch, ns[i], held);
+    auto read = [&](uint64_t at, uint64_t bytes) {
       at += body_off;
-      if (!dev || at + bytes <= host_copy[i].size()) return h[i] + at;
-      piece.resize(bytes);
-      return cudaMemcpy(piece.data(), ins[i] + at, bytes, cudaMemcpyDeviceToHost) == cudaSuccess ? piece.data() : nullptr;
+      return at + bytes <= held ? h[i] + at : window.read(at, bytes);
     };
     status[i] = parse_batches_from(read, ns[i] - body_off, nchunks, ph[i].batch, true, off[i], len[i], ph[i].wide);
-    if (status[i] == CUCM_ECUDA) return CUCM_ECUDA;
+    CK(fetched);
     if (!status[i]) ok.push_back(i);
   }
   // groups: one per unit length for model-free containers, one per prelearned container

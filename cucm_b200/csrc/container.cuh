@@ -237,8 +237,8 @@ inline int parse_header(const uint8_t *in, uint64_t n, Parsed &h) {
 // Chunk payload extents of the batches that follow the prelearn block
 // (cucm_decompress_v2.cu:1223-1237).  Offsets are relative to `body`.
 // read(off, n) gives n bytes of the body from `off` (inside it), or null when
-// they cannot be fetched; a batch's size field and its table are read, its
-// payloads are not.
+// they cannot be fetched; a batch's size field and its table are read, together,
+// its payloads are not.
 template <class Read>
 inline int parse_batches_from(Read read, uint64_t body_n, uint64_t nchunks, uint32_t batch, bool with_sizes,
                               std::vector<uint64_t> &off, std::vector<uint64_t> &len, bool wide) {
@@ -252,7 +252,7 @@ inline int parse_batches_from(Read read, uint64_t body_n, uint64_t nchunks, uint
     uint64_t bsz;
     if (with_sizes) {
       if (r + w > body_n) return CUCM_EFORMAT;
-      const uint8_t *size = read(r, w);
+      const uint8_t *size = read(r, std::min(w + w * C, body_n - r));
       if (!size) return CUCM_ECUDA;
       bsz = get_le(size, wide);
       r += w;
