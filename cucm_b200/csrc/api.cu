@@ -61,7 +61,10 @@ struct cucm_ctx {
   uint64_t launches = 0;
   uint64_t chunks = 0;
   bool timing_open = false;
+  LaunchForm launch;
 };
+
+LaunchForm cucm_last_launch(const cucm_ctx *c) { return c->launch; }
 
 namespace {
 
@@ -154,6 +157,7 @@ void timing_begin(cucm_ctx *c) {
   c->chunks = 0;
   c->kernel_ms = 0.0;
   c->kernel_pending = false;
+  c->launch = LaunchForm();
   cudaEventRecord(c->ev0, c->stream);
   c->timing_open = true;
 }
@@ -227,6 +231,8 @@ int run_engine(cucm_ctx *c, bool decode, std::vector<ChunkTask> &tasks, int unit
       tails = c->d_tails.as<TailTask>();
     }
     const uint8_t *img = ms.image ? c->image.as<uint8_t>() : nullptr;
+    c->launch.slots = std::max(c->launch.slots, grid);
+    if (decode) c->launch.decoder = decoder_form(grid, unit, cfg);
     CK(cudaEventRecord(c->evk0, c->stream));
     cudaError_t e = decode ? launch_decompress(c->d_tasks.as<ChunkTask>(), n, c->slots.as<uint8_t>(), grid, img,
                                                c->d_init.as<ModelInit>(), c->d_queue.as<uint32_t>(),
@@ -264,6 +270,8 @@ int run_engine(cucm_ctx *c, bool decode, std::vector<ChunkTask> &tasks, int unit
     for (uint32_t s = 0; s < S; s++) CK(cudaStreamWaitEvent(c->side[s], fork, 0));
     const uint8_t *img = ms.image ? c->image.as<uint8_t>() : nullptr;
     cfg.others = S - 1;
+    c->launch.slots = S;
+    if (decode) c->launch.decoder = decoder_form(1, unit, cfg);
     for (uint32_t i = 0; i < n; i++) {
       uint32_t s = i % S;
       uint8_t *slot = c->slots.as<uint8_t>() + (size_t)s * kSlotTableBytes;

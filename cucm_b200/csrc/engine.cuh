@@ -103,6 +103,23 @@ cudaError_t launch_fixed_encode(const FixedTask *d_tasks, const uint64_t *d_firs
 cudaError_t launch_fixed_decode(const FixedTask *d_tasks, uint32_t ntasks, const uint8_t *image,
                                 const ModelInit *d_init, uint32_t *d_queue, int sm_count, cudaStream_t stream);
 
+// The decoder's kernel for a launch of nslots chunks, and its shape.
+struct DecoderForm {
+  enum Kernel { kWide, kPairs, kGeneric } kernel;
+  int pairs;  // kPairs: chunks per CTA
+  bool low;   // kPairs: order 0/1 tables in shared memory
+  bool operator==(const DecoderForm &o) const { return kernel == o.kernel && pairs == o.pairs && low == o.low; }
+};
+DecoderForm decoder_form(uint32_t nslots, int unit, const EngineConfig &cfg);
+
+// What a context's last call came to: two calls on the same data, alike in form
+// and kernel choice, launch the same where these are the same.
+struct LaunchForm {
+  uint32_t slots = 0;  // chunks in flight, at most
+  DecoderForm decoder{DecoderForm::kGeneric, 0, false};
+  bool operator==(const LaunchForm &o) const { return slots == o.slots && decoder == o.decoder; }
+};
+
 size_t compress_smem_bytes(int unit);
 // Chunk slots of the engine that run at once on one SM.
 int engine_slots_per_sm(bool decode, int unit, const EngineConfig &cfg);
@@ -110,3 +127,6 @@ int compress_threads(int unit);
 size_t decompress_smem_bytes(int unit, int spec_bits);
 
 }  // namespace cucm
+
+struct cucm_ctx;
+cucm::LaunchForm cucm_last_launch(const cucm_ctx *ctx);

@@ -691,49 +691,54 @@ int engine_slots_per_sm(bool decode, int unit, const EngineConfig &cfg) {
   return smem > 110 * 1024 ? 1 : (smem > 72 * 1024 ? 2 : 3);
 }
 
+DecoderForm decoder_form(uint32_t nslots, int unit, const EngineConfig &cfg) {
+  if (!dec_fast(unit, cfg)) return {DecoderForm::kGeneric, 0, false};
+  int sms = cfg.sm_count;
+  if (sms <= 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) sms = 1;
+  }
+  // few chunks: an SM each (unless the caller chose a pair decoder's form)
+  if (nslots + cfg.others <= kWideMaxChunks && nslots <= (uint32_t)sms && cfg.dec_pairs == 0 && cfg.dec_tables == 0)
+    return {DecoderForm::kWide, 0, true};
+  // One chunk per warp pair; spread the pairs over all SMs before stacking them.
+  int wpc = (int)((nslots + (uint32_t)sms - 1) / (uint32_t)sms);
+  if (cfg.dec_pairs > 0) wpc = cfg.dec_pairs;
+  wpc = std::max(1, std::min(wpc, dec_max_pairs(unit)));
+  // a chunk alone in its CTA keeps its order 0/1 tables in shared memory
+  // (two would fit, but a fourth gather costs less than their lookups take
+  // from the load/store pipe: 64 MiB in 256 chunks, 722 ms from HBM, 731)
+  const bool low = cfg.dec_tables == 0 && wpc == 1 && make_dec_layout(unit, wpc, true).total <= kDecSmemLimit;
+  return {DecoderForm::kPairs, wpc, low};
+}
+
 cudaError_t launch_decompress(const ChunkTask *d_tasks, uint32_t ntasks, uint8_t *slots, uint32_t nslots,
                               const uint8_t *init_tables, const ModelInit *d_init, uint32_t *d_queue,
                               uint32_t *d_status, const EngineConfig &cfg, cudaStream_t stream, int unit) {
-  if (dec_fast(unit, cfg)) {
-    // One chunk per warp pair; spread the pairs over all SMs before stacking them.
-    int sms = cfg.sm_count;
-    if (sms <= 0) {
-      int dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      if (sms <= 0) sms = 1;
-    }
-    const uint32_t spin = cfg.spin_limit ? cfg.spin_limit : kDecSpinLimit;
-    // few chunks: an SM each (unless the caller chose a pair decoder's form)
-    if (nslots + cfg.others <= kWideMaxChunks && nslots <= (uint32_t)sms && cfg.dec_pairs == 0 && cfg.dec_tables == 0) {
-      const DecLayout L = make_dec_layout(unit, 1, true);
-      cudaError_t e = set_smem((const void *)decompress_wide_kernel, L.total);
-      if (e != cudaSuccess) return e;
-      decompress_wide_kernel<<<nslots, kWideThreads, L.total, stream>>>(d_tasks, ntasks, slots, init_tables, d_init,
-                                                                        d_queue, d_status, unit, spin);
-      return cudaGetLastError();
-    }
-    int wpc = (int)((nslots + (uint32_t)sms - 1) / (uint32_t)sms);
-    const int wmax = dec_max_pairs(unit);
-    if (cfg.dec_pairs > 0) wpc = cfg.dec_pairs;
-    if (wpc > wmax) wpc = wmax;
-    if (wpc < 1) wpc = 1;
-    // a chunk alone in its CTA keeps its order 0/1 tables in shared memory
-    // (two would fit, but a fourth gather costs less than their lookups take
-    // from the load/store pipe: 64 MiB in 256 chunks, 722 ms from HBM, 731)
-    const DecLayout Low = make_dec_layout(unit, wpc, true);
-    const bool low = cfg.dec_tables == 0 && wpc == 1 && Low.total <= kDecSmemLimit;
-    const DecLayout L = low ? Low : make_dec_layout(unit, wpc);
-    const void *kern = low ? (const void *)decompress_pair_kernel<true> : (const void *)decompress_pair_kernel<false>;
+  const DecoderForm f = decoder_form(nslots, unit, cfg);
+  const uint32_t spin = cfg.spin_limit ? cfg.spin_limit : kDecSpinLimit;
+  if (f.kernel == DecoderForm::kWide) {
+    const DecLayout L = make_dec_layout(unit, 1, true);
+    cudaError_t e = set_smem((const void *)decompress_wide_kernel, L.total);
+    if (e != cudaSuccess) return e;
+    decompress_wide_kernel<<<nslots, kWideThreads, L.total, stream>>>(d_tasks, ntasks, slots, init_tables, d_init,
+                                                                      d_queue, d_status, unit, spin);
+    return cudaGetLastError();
+  }
+  if (f.kernel == DecoderForm::kPairs) {
+    const DecLayout L = make_dec_layout(unit, f.pairs, f.low);
+    const void *kern = f.low ? (const void *)decompress_pair_kernel<true> : (const void *)decompress_pair_kernel<false>;
     cudaError_t e = set_smem(kern, L.total);
     if (e != cudaSuccess) return e;
-    const uint32_t grid = (nslots + (uint32_t)wpc - 1) / (uint32_t)wpc;
-    if (low)
-      decompress_pair_kernel<true><<<grid, wpc * 64, L.total, stream>>>(d_tasks, ntasks, slots, nslots, init_tables,
-                                                                        d_init, d_queue, d_status, unit, spin);
+    const uint32_t grid = (nslots + (uint32_t)f.pairs - 1) / (uint32_t)f.pairs;
+    if (f.low)
+      decompress_pair_kernel<true><<<grid, f.pairs * 64, L.total, stream>>>(
+          d_tasks, ntasks, slots, nslots, init_tables, d_init, d_queue, d_status, unit, spin);
     else
-      decompress_pair_kernel<false><<<grid, wpc * 64, L.total, stream>>>(d_tasks, ntasks, slots, nslots, init_tables,
-                                                                         d_init, d_queue, d_status, unit, spin);
+      decompress_pair_kernel<false><<<grid, f.pairs * 64, L.total, stream>>>(
+          d_tasks, ntasks, slots, nslots, init_tables, d_init, d_queue, d_status, unit, spin);
     return cudaGetLastError();
   }
   size_t smem = decompress_smem_bytes(unit, cfg.spec_bits);

@@ -275,7 +275,9 @@ int cucm_last_launches(cucm_ctx *ctx, uint64_t *n);
  * times each (>= 1; the fastest repetition counts), checks that every
  * candidate gives the same container and gives the sample back (else
  * CUCM_EMISMATCH), then applies to the context and writes to *best the
- * choice with the least compress + decompress device time.  The other
+ * choice with the least compress + decompress device time.  Candidates that
+ * come to the same launch share their fastest time, and of those the derived
+ * rule (0, for cmp_ctas the most that fit) is taken.  The other
  * tuning fields are kept.  results (may be null) receives up to `cap`
  * measured candidates, *count their number.  A sample with the target
  * workload's number of chunks gives choices that carry over to it. */
