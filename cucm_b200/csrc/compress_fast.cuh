@@ -62,7 +62,6 @@ typedef Tables FastTables;
 // orders' rows start in different banks.
 constexpr int kStatePad = 16, kSortPad = 8;
 constexpr int kRecRow = 257;   // 256 states: the rows start in different banks, bits of one order spread over all
-constexpr int kChainRow = 37;  // 32 steps and 4 of read-ahead; odd, so that the rows start in different banks
 
 constexpr uint32_t kUntouched = 0xffu;  // no state: the largest is 252
 constexpr int kClaimLog = 9, kClaim = 1 << kClaimLog;  // places of a claim table
@@ -70,12 +69,12 @@ constexpr int kClaimLog = 9, kClaim = 1 << kClaimLog;  // places of a claim tabl
 struct FastLayout {
   int U, NSLOT, stage;
   int ks, ls;   // row lengths of key and of lnk / bkt
-  size_t off_tab, off_rec, off_w, off_claim, off_late, off_ns, off_key, off_lnk, off_bkt, off_fsw, off_st, off_srt, off_step,
+  size_t off_tab, off_rec, off_w, off_claim, off_late, off_ns, off_key, off_lnk, off_bkt, off_fsw, off_st, off_srt,
       off_fr, off_yw, off_c1, off_prm, off_win, off_stage, total;
 };
 
-__host__ __device__ inline FastLayout make_fast_layout(int U) {
-  FastLayout L;
+__host__ __device__ constexpr FastLayout make_fast_layout(int U) {
+  FastLayout L{};
   L.U = U;
   L.NSLOT = U <= 128 ? 128 : 256;  // slots per order and unit
   L.ks = U + 4;  // rows of 8 orders that start in different banks
@@ -101,7 +100,6 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
   L.off_fsw = take((size_t)2 * kOrders * U);               // gathered slot states
   L.off_st = take((size_t)kOrders * (U + kStatePad));      // live state [order][bit]
   L.off_srt = take(sizeof(uint16_t) * 2 * kOrders * (U + kSortPad));  // updates grouped by state [unit parity][order]
-  L.off_step = take((size_t)16 * kOrders * kChainRow);     // operands of 32 updates [order]
   L.off_fr = take((size_t)2 * U * kOrders);                // frozen state
   L.off_yw = take(sizeof(uint32_t) * 4 * (U / 32));        // bits, by unit mod 4
   L.off_c1 = take((size_t)4 * (U / 8));                    // previous byte per byte, by unit mod 4
@@ -112,7 +110,12 @@ __host__ __device__ inline FastLayout make_fast_layout(int U) {
   return L;
 }
 
-struct ChainStep;
+// Shared memory that a CTA takes of its SM's 228 KiB, 1 KiB of it reserved by
+// the hardware.  Two CTAs share an SM at every unit: 2 * 110,032 of 233,472
+// bytes at 256 bits.
+constexpr size_t kFastSmBytes = 228 * 1024;
+__host__ __device__ constexpr size_t fast_sm_bytes(int U) { return make_fast_layout(U).total + 1024 + 64; }
+static_assert(2 * fast_sm_bytes(kFastMaxUnit) <= kFastSmBytes, "two CTAs an SM");
 
 struct FastSmem {
   FastTables *tab;
@@ -127,7 +130,6 @@ struct FastSmem {
   uint8_t *fsw;      // [2][U][8]
   uint8_t *st;       // [8][U + kStatePad]
   uint16_t *srt;     // [2][8][U + kSortPad]
-  ChainStep *step;    // [8][kChainRow]
   uint8_t *fr;       // [2][U][8]
   uint32_t *yw;      // [4][U/32]
   uint8_t *c1;       // [4][U/8]
@@ -150,7 +152,6 @@ __device__ inline FastSmem carve_fast(uint8_t *b, const FastLayout &L) {
   s.fsw = b + L.off_fsw;
   s.st = b + L.off_st;
   s.srt = reinterpret_cast<uint16_t *>(b + L.off_srt);
-  s.step = reinterpret_cast<ChainStep *>(b + L.off_step);
   s.fr = b + L.off_fr;
   s.yw = reinterpret_cast<uint32_t *>(b + L.off_yw);
   s.c1 = b + L.off_c1;

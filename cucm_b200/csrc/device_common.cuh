@@ -8,12 +8,12 @@
 constexpr int kStageMin = 4096;
 constexpr uint32_t kFlushBlock = 512;
 
-__host__ __device__ inline int next_pow2(int v) {
+__host__ __device__ constexpr int next_pow2(int v) {
   int p = 1;
   while (p < v) p <<= 1;
   return p;
 }
-__host__ __device__ inline int ilog2(int v) {
+__host__ __device__ constexpr int ilog2(int v) {
   int l = 0;
   while ((1 << l) < v) l++;
   return l;

@@ -624,12 +624,10 @@ cudaError_t upload_tables() {
   return cudaMemcpyToSymbol(g_tables, &t, sizeof(Tables));
 }
 
-// Pipelined compressor CTAs that fit on one SM: shared memory (1 KiB of it
-// reserved per CTA by the hardware) and the registers of two CTAs
-// (__launch_bounds__(kFastThreads, 2)).
+// Pipelined compressor CTAs that fit on one SM: shared memory and the registers
+// of two CTAs (__launch_bounds__(kFastThreads, 2)).
 static int fast_ctas_per_sm(int unit) {
-  const size_t per = make_fast_layout(unit).total + 1024 + 64;
-  const int by_smem = (int)((228u * 1024u) / per);
+  const int by_smem = (int)(kFastSmBytes / fast_sm_bytes(unit));
   const int by_regs = 2;
   const int n = by_smem < by_regs ? by_smem : by_regs;
   return n < 1 ? 1 : n;
