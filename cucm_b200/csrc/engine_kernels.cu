@@ -588,6 +588,10 @@ cudaError_t launch_fixed_encode(const FixedTask *d_tasks, const uint64_t *d_firs
     if (e != cudaSuccess) return e;
   }
   const int lanes = coder_lanes(ntasks, sm_count);
+  if (lanes == 1) {
+    fixed_coder_warp_kernel<<<ntasks, 32, 0, stream>>>(d_tasks, d_status);
+    return cudaGetLastError();
+  }
   fixed_coder_kernel<<<(ntasks + lanes - 1) / lanes, 32, 0, stream>>>(d_tasks, ntasks, d_status, lanes);
   return cudaGetLastError();
 }

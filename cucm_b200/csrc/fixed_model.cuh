@@ -21,7 +21,9 @@
 //                       coder inputs (pr << 1 | y) -- every bit of every
 //                       chunk in parallel -- into a u16 array;
 //   fixed_coder_kernel  one thread per chunk runs the arithmetic coder over
-//                       its chunk's array;
+//                       its chunk's array, or, while every chunk can have a
+//                       warp scheduler of its own, a warp
+//                       (fixed_coder_warp_kernel);
 //
 // and the decoder gives each chunk a warp, a nibble per round, or in calls with
 // no more chunks than SMs a CTA, a byte per round.
@@ -114,11 +116,49 @@ CUCM_UNROLL
   }
 }
 
+// Warp = task: the coder as in the adaptive compressor, all lanes alike.  The
+// lanes turn 32 bytes' inputs into the coder's entries side by side and write
+// the bytes out together; a thread that does both beside its chain of bits is
+// bound by the instructions it issues and takes 78 cycles a bit against 53, more
+// than the 71 of a test after every bit.  Text, both kernels of the variant, ms
+// with a test after every bit / a thread / a warp: one chunk of 64 KiB 19.1 /
+// 20.9 / 13.9, 128 chunks of 16 KiB 9.1 / 6.4 / 4.6.
+constexpr int kFixedStage = 2048;  // 32 bytes code at most 1 KiB; flushes go out in 512-byte blocks
+
+__global__ void __launch_bounds__(32)
+    fixed_coder_warp_kernel(const FixedTask *tasks, uint32_t *status) {
+  __shared__ uint4 ent[32 * 4];
+  __shared__ __align__(16) uint8_t stage[kFixedStage];
+  const int lane = threadIdx.x;
+  const FixedTask t = tasks[blockIdx.x];
+  const uint4 *src = reinterpret_cast<const uint4 *>(t.prm);
+  const uint64_t n = t.in_len;
+  Coder c{0u, 0xffffffffu, 0, 0};
+  auto load = [&](uint64_t p) { return p + lane < n ? __ldg(src + p + lane) : make_uint4(0, 0, 0, 0); };
+  uint4 next = load(0);
+  for (uint64_t p = 0; p < n; p += 32) {
+    const uint32_t w[4] = {next.x, next.y, next.z, next.w};
+CUCM_UNROLL
+    for (int i = 0; i < 4; i++) {
+      const uint2 a = coder_entry(w[i] & 0xffffu), b = coder_entry(w[i] >> 16);
+      ent[4 * lane + i] = make_uint4(a.x, a.y, b.x, b.y);
+    }
+    next = load(p + 32);
+    __syncwarp();
+    const int bytes = n - p < 32 ? (int)(n - p) : 32;
+    coder_run_p(c, reinterpret_cast<const uint2 *>(ent), stage, kFixedStage, 8 * bytes);
+    coder_flush_p(c, stage, kFixedStage, t.out, t.out_cap);
+  }
+  coder_finish_p(c, stage, kFixedStage, t.out, t.out_cap, t.result);
+  if (lane == 0 && c.head > t.out_cap) atomicOr(status, (uint32_t)kDevOverflow);
+}
+
 // Thread = task: the binary coder over the chunk's coder inputs, two bytes'
 // (16 bits, one coder_group) at a time, then the flush byte
 // (cucm_compress_v2.cu:902) and the payload length.  The next two bytes'
-// inputs are in flight while two are coded.  16 MiB of text in 128 chunks,
-// both kernels of the variant: 72 -> 51 ms against a test after every bit.
+// inputs are in flight while two are coded.  For more chunks than warp
+// schedulers: 600 of 16 KiB of text, both kernels, 13.0 -> 10.4 ms against a
+// test after every bit.
 __global__ void __launch_bounds__(32) fixed_coder_kernel(const FixedTask *tasks, uint32_t ntasks, uint32_t *status,
                                                          int lanes) {
   __shared__ uint8_t rings[32 * (kLaneRing + 4)];
