@@ -594,6 +594,20 @@ __device__ __forceinline__ uint32_t dec_ahead(DecCoder &c, uint8_t *win, const u
   return dec_next4(win, (uint32_t)((long long)c.ioff - c.wbase));
 }
 
+// The bounded waits of a chunk's warps for one another.
+template <class There, class Then>
+__device__ __forceinline__ bool dec_wait(There there, uint32_t limit, Then then) {
+  auto fenced = [&] {
+    __threadfence_block();
+    then();
+  };
+  return warp_wait(there, [](bool x) { return __all_sync(0xffffffffu, x) != 0; }, limit, fenced);
+}
+template <class There>
+__device__ __forceinline__ bool dec_wait(There there, uint32_t limit) {
+  return dec_wait(there, limit, [] {});
+}
+
 // The byte after `hist` joins it.
 __device__ __forceinline__ void dec_push(uint32_t hist[7], uint32_t byte) {
 CUCM_UNROLL
@@ -630,13 +644,9 @@ __device__ void decompress_pair_one(const ChunkTask &t, uint8_t *slot, const Dec
     for (uint64_t base = 0; base < nbits; base += (uint64_t)U) {
       const int nunit = (int)(nbits - base < (uint64_t)U ? nbits - base : (uint64_t)U);
       for (int rd = 0; rd < (nunit >> 2); rd++) {
-        uint32_t spins = 0;
-        while (ok && s.prog[0] <= done) {
-          // a plain poll: a sleep here wakes late and the updating warp
-          // falls rounds behind by the unit's end
-          if (++spins >= spin_limit) ok = false;
-        }
-        __threadfence_block();
+        // a plain poll: a sleep here wakes late and the updating warp
+        // falls rounds behind by the unit's end
+        ok = ok && dec_wait([&] { return s.prog[0] > done; }, spin_limit);
         if (!ok) break;
         dec_update_round(s, tab, L, lane, rd);
         done++;

@@ -116,22 +116,18 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
         dec_settle(c, path, s.win);
         next = dec_ahead(c, s.win, pay, plen, lane);
         // the predictions below it
-        uint32_t spins = 0, have;
-        while ((have = ready[hi]) != seq + 1 && have != seq + 2) {
-          if (!ok || ++spins >= spin_limit) {
-            ok = false;
-            break;
-          }
-        }
-        __threadfence_block();
-        uint32_t f_node = ws.f[hi][lane & 15];
-        if (have != seq + 1) {  // not followed, and there it is
+        uint32_t have, f_node;
+        const bool seen = dec_wait([&] { return (have = ready[hi]) == seq + 1 || have == seq + 2; },
+                                   ok ? spin_limit : 1, [&] { f_node = ws.f[hi][lane & 15]; });
+        ok = ok && seen;
+        const bool followed = seen && have == seq + 1;
+        if (!followed) {  // not followed, and there it is
           ln.gather(hi, 4, hist, kk, st);
           pr = ln.predict(s, tab->squash, st, hist[0], smp, cxt);
           f_node = pr << 20;
         }
         const uint32_t lo = dec_nibble(c, path, f_node, next, s.win, lane);
-        if (have != seq + 1) dec_write_record(s, ln, dec_record(ln, kk, st, smp, pr, cxt, lo), 2 * b + 1);
+        if (!followed) dec_write_record(s, ln, dec_record(ln, kk, st, smp, pr, cxt, lo), 2 * b + 1);
         const uint32_t byte = (hi << 4) | lo;
         if (lane == 0) ws.byte[nth % kWidePlaces] = byte;
         __syncwarp();
@@ -186,11 +182,7 @@ __device__ void decompress_wide_one(const ChunkTask &t, uint8_t *slot, const Dec
       for (int rd = 0; rd < (nunit >> 2); rd++) {
         const uint32_t done = bytes + (uint32_t)(rd >> 1);
         volatile uint32_t *prog = s.prog + (rd & 1 ? 2 : 0);
-        uint32_t spins = 0;
-        while (ok && (int32_t)(*prog - done) <= 0) {
-          if (++spins >= spin_limit) ok = false;
-        }
-        __threadfence_block();
+        ok = ok && dec_wait([&] { return (int32_t)(*prog - done) > 0; }, spin_limit);
         if (!ok) break;
         dec_update_round(s, tab, L, lane, rd);
       }

@@ -27,6 +27,7 @@
 #include "engine.cuh"
 #include "model.cuh"
 #include "tables.h"
+#include "warp_wait.h"
 #include "wide_crossing.h"
 
 namespace cucm {

@@ -321,8 +321,10 @@ __global__ void __launch_bounds__(kFixedWideThreads, 1)
         const uint32_t hi = dec_nibble(c, path, pr << 20, next, win, lane);
         dec_settle(c, path, win);
         next = dec_ahead(c, win, t.in, t.in_len, lane);
-        // ends with its warp's gathers; past the bound the nibble is predicted
-        // here, with the same result, so there is nothing to report
+        // ends with its warp's gathers, long before the bound; past it the nibble
+        // is predicted here, with the same result, so there is nothing to report.
+        // (No vote on the outcome, as warp_wait takes where a caller can set the
+        // bound: 2 % of this kernel, 16.2 -> 16.6 ms for 8 KiB of random bytes.)
         uint32_t spins = 0, have;
         while ((have = ready[hi]) != seq + 1 && have != seq + 2)
           if (++spins >= kDecSpinLimit) break;
