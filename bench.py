@@ -33,7 +33,8 @@ Other workloads (one JSON line each, not the headline):
 --impl reference times the reference's own implementation of the path on the
 host cores: its two programs built for the CPU from its unmodified sources
 (oracle/_ref), one chunk per process on all cores, on a bounded sample of
-the same workload.  Under torchrun, rank 0 alone runs it.
+the same workload.  Under torchrun, rank 0 alone runs it.  Where those programs
+are not built it says so and times nothing in their place.
 
 Multi-GPU (--gpus N; started under torchrun by the script itself when run
 alone): one process per GPU, one stream of N x 256 MiB split into
@@ -275,6 +276,10 @@ def headline_config():
 
 def run_reference(args, rank, world):
     if rank != 0:
+        return
+    if _ref_bins()[2] != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's programs are not built here (oracle/_ref)"}),
+              flush=True)
         return
     from cucm_b200 import workloads as W
     data, _ = W.config1()
