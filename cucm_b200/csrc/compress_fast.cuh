@@ -112,7 +112,9 @@ __host__ __device__ constexpr FastLayout make_fast_layout(int U) {
 
 // Shared memory that a CTA takes of its SM's 228 KiB, 1 KiB of it reserved by
 // the hardware.  Two CTAs share an SM at every unit: 2 * 110,032 of 233,472
-// bytes at 256 bits.
+// bytes at 256 bits.  What they leave is L1, in steps: at 128 bits two take 160
+// KB, and 4.7 KB more a CTA moved the split from 164 to 196 KB: 128 MiB in 256
+// chunks 348 -> 362 ms (it may be that gathers in flight hold L1 lines).
 constexpr size_t kFastSmBytes = 228 * 1024;
 __host__ __device__ constexpr size_t fast_sm_bytes(int U) { return make_fast_layout(U).total + 1024 + 64; }
 static_assert(2 * fast_sm_bytes(kFastMaxUnit) <= kFastSmBytes, "two CTAs an SM");
@@ -230,11 +232,13 @@ __device__ __forceinline__ void front_keys(const FastSmem &s, const FastLayout &
 // key's claim go on to a second table.  Nothing is cleared: a place is only
 // read by bits that have just written it, and the previous unit's tables only
 // lead to a position whose key is compared.  With 4 places per bit (units of
-// 128 bits), 12 % of the keys need the second table and one in ~600 neither
-// claim: those are numbered one after the other and listed.  The two orders' ~12 shared-memory steps take
-// 3,250 cycles a unit of 128 bits for a CTA alone; sorting each order's keys
-// across the warp and searching the rows took 8,100 of the front warps'
-// 12,000.
+// 128 bits), 10-11 % of the keys of text, walk and random bytes need the second
+// table and one in ~700 gets neither: those are numbered one after the other and
+// listed.  At 2 places per bit (256 bits) it is 20 % and one in ~100, 18 of a
+// unit's 2,048; tables twice as long take 16 KB more, and two CTAs would not fit an SM.  The
+// two orders' ~12 shared-memory steps take 3,250 cycles a unit of 128 bits for a
+// CTA alone; sorting each order's keys across the warp and searching the rows
+// took 8,100 of the front warps' 12,000.
 //
 // Front warp w owns orders 2w and 2w + 1, so no other warp writes their
 // tables.  E bits per lane: 32 * E >= U.
@@ -918,7 +922,8 @@ __global__ void __launch_bounds__(kFastThreads, 2)
   compress_fast_loop<8>(tasks, ntasks, slots, init_tables, init, queue, status, unit, tails, tail_count, roles);
 }
 
-// Units of 160..256 bits.
+// Units of 160..256 bits: 16 gathers a thread, 44 bytes spilled at the 128
+// registers of two CTAs.
 __global__ void __launch_bounds__(kFastThreads, 2)
     compress_fast_kernel_wide(const ChunkTask *tasks, uint32_t ntasks, uint8_t *slots, const uint8_t *init_tables,
                               const ModelInit *init, uint32_t *queue, uint32_t *status, int unit, TailTask *tails,

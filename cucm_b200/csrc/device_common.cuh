@@ -98,8 +98,10 @@ __device__ __forceinline__ void coder_step(const uint2 &q, uint32_t &x1, uint32_
 // byte goes to the ring's head whether or not the head then advances past it.
 // A bit that has to shift out two bytes or more (coded against odds of 2^8
 // and up) is seen in `least`, and its group is done again in the reference's
-// form.  48 cycles a bit for a warp alone against 80-90 with the test after
-// every bit, whatever the data; 8 bits a group measured 50, 4 bits 62, groups
+// form.  48 cycles a bit for a warp alone (a probe; 50 in the compressor's coder
+// warp, 53 in the fixed-model coder's; 62 in the tail pass, whose one thread a
+// chunk votes and writes its bytes too) against 80-90 with the test after every
+// bit, whatever the data; 8 bits a group measured 50, 4 bits 62, groups
 // tested as a whole and resumed after the first shift 42-56, a next product
 // for either outcome of the test 46-52, shifts of two bytes in the group as
 // well 17 % more.  get(k) is the group's entry k in
